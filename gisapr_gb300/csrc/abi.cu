@@ -54,7 +54,7 @@ cudaError_t launch_packed_ctf(cudaStream_t, const float*, const float*, const fl
                               float, float, float, float, float*);
 size_t prepare_scratch_elems(int N, int nb);
 cudaError_t launch_prepare_particles(cudaStream_t, const float*, int, int, const int*, const void*,
-                                     const float*, const float*, float2*, float2*, int,
+                                     const float*, const float*, float2*, float2*, int, int,
                                      const float2*, const float2*, int, int);
 int correlate_cluster_size(int n);
 size_t correlate_smem_bytes(int n, int n_psi, int crop, int cluster);
@@ -621,11 +621,11 @@ int gisapr_prepare_particles(gisapr_ctx ctx, void* stream, const float* images, 
   if (rc) return rc;
   const int grid = grid_for(ctx, n * n_psi, 4);
   rc = ensure(ctx, ctx->prep_scratch, (size_t)grid * prepare_scratch_elems(box, newbox) * sizeof(float2),
-              "cudaMalloc(particle scratch)");
+              "cudaMalloc(particle scratch)");  // nothing below box 256
   if (rc) return rc;
   GISAPR_CHECK_CUDA(launch_prepare_particles((cudaStream_t)stream, images, n, n_psi, psi_index, psi_table, mask,
-                                             ctf, (float2*)out, (float2*)ctx->prep_scratch.ptr, grid, ctx->tw, ctx->tw3,
-                                             box, newbox),
+                                             ctf, (float2*)out, (float2*)ctx->prep_scratch.ptr, grid, ctx->sm_count,
+                                             ctx->tw, ctx->tw3, box, newbox),
                     "prepare_particles");
   return GISAPR_OK;
 }

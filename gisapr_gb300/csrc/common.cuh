@@ -14,8 +14,50 @@
 // Largest 1-D transform length any kernel stages in shared memory.
 constexpr int kMaxFftLen = 512;
 
-GISAPR_DEV float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-GISAPR_DEV float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// Packed float32 pairs (PTX f32x2): one instruction for both halves, each
+// rounded as its scalar form. The FMA pipes do as many operations a cycle as
+// with scalar instructions (measured on GB300: 39.3 against 38.3 T a second),
+// so what a pair saves is issue slots: complex sums in this form took 1% to 3%
+// off the kernels that are made of FFT codelets.
+GISAPR_DEV unsigned long long f2_bits(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+GISAPR_DEV float2 f2_of(unsigned long long a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+GISAPR_DEV float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+}
+GISAPR_DEV float2 sub2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+}
+GISAPR_DEV float2 mul2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+}
+GISAPR_DEV float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c)));
+  return f2_of(r);
+}
+GISAPR_DEV float2 add2_down(float2 a, float2 b) {  // rounded towards minus infinity
+  unsigned long long r;
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+}
+GISAPR_DEV float2 dup2(float a) { return make_float2(a, a); }
+
+GISAPR_DEV float2 cadd(float2 a, float2 b) { return add2(a, b); }
+GISAPR_DEV float2 csub(float2 a, float2 b) { return sub2(a, b); }
 GISAPR_DEV float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }

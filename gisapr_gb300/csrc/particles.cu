@@ -7,12 +7,14 @@
 // fused multiply-add, because gamma reaches hundreds of radians and a single
 // rounding difference moves sin(gamma) by ~1e-5.
 //
-// prepare_particles: one CTA per (particle, psi). Rows of the rotated image
-// (bilinear, zero padding, align_corners=True, in the weight order of
-// torch's vectorised 2-D CPU kernel) are masked and transformed in shared
-// memory, then columns; the packed half plane is Fourier-cropped, multiplied
-// by the CTF table, conjugated, L2-normalised and written pre-shifted.
+// prepare_plane (boxes up to 192): the rotated image (bilinear, zero padding,
+// align_corners=True, in the weight order of torch's vectorised 2-D CPU kernel)
+// is masked and transformed in one shared-memory plane; the packed half plane
+// is Fourier-cropped, multiplied by the CTF table, conjugated, L2-normalised
+// and written pre-shifted. prepare_particles does the same for box 256, whose
+// plane does not fit an SM, through a global scratch plane.
 #include "common.cuh"
+#include "pairplane.cuh"
 
 namespace {
 
@@ -173,6 +175,236 @@ __global__ void __launch_bounds__(kThreads) prepare_particles(PrepParams P) {
   }
 }
 
+
+// ---------------------------------------------------------------------------
+// Boxes 32 to 192: one image per CTA and pass, all of it in shared memory.
+//
+// The image is rotated straight into the pair plane (pairplane.cuh), so a
+// spectrum costs one write and one read of the plane per FFT step and one
+// write to HBM, against the block-wide radix-2 transforms through a global
+// scratch plane that prepare_particles runs (box 128: each of 14 stages a pass
+// over shared memory with a block barrier, and three passes over the scratch).
+// Measured on GB300, 2,000 particles of box 128 at three angles: 2.51 -> 0.75 ms
+// (597 MB of images, weights and spectra, 0.8 TB/s). What bounds it now is issue
+// and latency at 16 warps an SM: about 35 packed instructions a pixel for the
+// float32 coordinate chain and the bilinear sum, and the FFT codelets.
+//
+// Up to box 128 the source image is staged in shared memory, with a border of
+// two zero pixels that stands for the zero padding (coordinates are clamped
+// into the border), because a rotated footprint touches about ten 128-byte
+// lines per warp load, which the L1 serves one a cycle; the row stride of
+// N + 9 spreads the footprint over the banks. A CTA takes a contiguous run of
+// (particle, psi) jobs, so an image is loaded once for its psi angles; at box
+// 128, where one CTA fills the SM, the next image arrives by asynchronous
+// copies meanwhile. Box 192 has no room for the image and samples it through L1.
+// ---------------------------------------------------------------------------
+template <int N>
+__host__ __device__ constexpr int prep_threads() { return N <= 64 ? 128 : (N == 96 ? 384 : (N == 128 ? 512 : 768)); }
+template <int N>
+__host__ __device__ constexpr int prep_images() { return N == 128 ? 2 : (N < 128 ? 1 : 0); }
+constexpr int kBorder = 2;
+template <int N>
+__host__ __device__ constexpr int image_ld() { return N + 9; }
+template <int N>
+__host__ __device__ constexpr int image_elems() { return (N + 2 * kBorder) * image_ld<N>(); }
+
+// a / (N - 1), correctly rounded: one Newton correction of a * RN(1 / (N - 1))
+// (Markstein's theorem; the remainder is exact in the fused multiply-add).
+template <int N>
+__device__ __forceinline__ float2 div_nm1(float2 a) {
+  constexpr float d = (float)(N - 1), r = 1.0f / (float)(N - 1);
+  const float2 q = mul2(a, dup2(r));
+  return fma2(fma2(q, dup2(-d), a), dup2(r), q);
+}
+
+// s + c += x * x in two floats (48 bits): GB300's FP64 rate is 1/64 of its
+// FP32 rate, and the L2 norm's FP64 sums took as long as the transforms.
+__device__ __forceinline__ void add_square(float x, float& s, float& c) {
+  const float t = __fmaf_rn(x, x, s);
+  c = __fadd_rn(c, __fmaf_rn(x, x, -__fsub_rn(t, s)));
+  s = t;
+}
+
+__device__ __forceinline__ float small_to_float(int i) {  // 0 <= i < 2^23, FP32 pipe
+  return __int_as_float(0x4B000000 | i) - 8388608.0f;
+}
+
+template <int N>
+__global__ void __launch_bounds__(prep_threads<N>(), N <= 64 ? 4 : (N == 96 ? 2 : 1)) prepare_plane(PrepParams P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int NT = prep_threads<N>(), NW = NT / 32, G = fft_lines<N>(), NI = prep_images<N>();
+  constexpr int ILD = image_ld<N>(), IEL = image_elems<N>();
+  float2* plane = reinterpret_cast<float2*>(smem_raw);
+  float2* s_tw = plane + pair_elems(N);
+  float2* s_last = s_tw + N;                              // [N] the Nyquist column, then packed column nb / 2
+  double* red = reinterpret_cast<double*>(s_last + N);    // [NW + 1]
+  float* s_img = reinterpret_cast<float*>(red + NW + 1);  // [NI][IEL]
+  const PairPlane<N> Z{plane};
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nb = P.nb, H = nb / 2 + 1;
+  for (int t = tid; t < N; t += NT) s_tw[t] = twiddle_of<N>(P.tw, P.tw3, t);
+  for (int t = tid; t < NI * IEL; t += NT) s_img[t] = 0.f;  // the border stays zero
+  const long long jobs = (long long)P.n * P.n_psi;
+  const int j0 = (int)(jobs * blockIdx.x / gridDim.x), j1 = (int)(jobs * (blockIdx.x + 1) / gridDim.x);
+  // the images of particles p0 .. p1 go to the buffers in turn
+  const int p0 = j0 / P.n_psi, p1 = j1 > j0 ? (j1 - 1) / P.n_psi : p0 - 1;
+  auto load_image = [&](int p) {
+    if constexpr (NI > 0) {
+      float* dst = s_img + ((p - p0) % NI) * IEL + kBorder * ILD + kBorder;
+      const float* src = P.images + (size_t)p * N * N;
+      for (int t = tid; t < N * N; t += NT)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(dst + (t / N) * ILD + t % N)),
+                     "l"(src + t)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  __syncthreads();  // the zeroed border before the copies
+  if (NI > 0 && p0 <= p1) load_image(p0);
+  int ready = p0 - 1;  // the last image that has been waited for
+  const float half = __fdiv_rn((float)(N - 1), 2.0f);
+  // lanes take 8 columns x 4 row pairs of the rotated image: a compact footprint
+  const int lj = tid & 7, lq = (tid >> 3) & 3;
+  constexpr int JT = N / 8, QT = N / 8;  // tiles of 8 columns, of 4 row pairs
+  for (int job = j0; job < j1; ++job) {
+    const int p = job / P.n_psi, si = job - p * P.n_psi;
+    if (NI > 0 && p != ready) {
+      if (NI > 1 && p + 1 <= p1) {
+        load_image(p + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        if (NI == 1 && p != p0) load_image(p);  // every reader left it at the last barrier
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      ready = p;
+      __syncthreads();
+    }
+    const float4 ps = P.psi_tab[P.psi_index[(size_t)p * P.n_psi + si]];
+    const float cth = ps.x, sth = ps.y;
+    const float* img = NI > 0 ? s_img + (NI > 1 ? ((p - p0) % NI) * IEL : 0) : P.images + (size_t)p * N * N;
+#pragma unroll 2
+    for (int tile = warp; tile < JT * QT; tile += NW) {
+      // the two rows of a pair, as the halves of packed operations
+      const int q = (tile / JT) * 4 + lq, j = (tile % JT) * 8 + lj;
+      const float xx = small_to_float(j), y0f = small_to_float(2 * q);
+      const float2 yy = make_float2(y0f, y0f + 1.0f);
+      // source = [row, col] @ M^T + offset; M = [[c, -s], [s, c]]
+      const float2 sy = add2(fma2(dup2(-sth), dup2(xx), mul2(dup2(cth), yy)), dup2(ps.z));
+      const float2 sx = add2(fma2(dup2(cth), dup2(xx), mul2(dup2(sth), yy)), dup2(ps.w));
+      const float2 yn = add2(div_nm1<N>(mul2(dup2(2.0f), sy)), dup2(-1.0f));
+      const float2 xn = add2(div_nm1<N>(mul2(dup2(2.0f), sx)), dup2(-1.0f));
+      const float2 iy = mul2(add2(yn, dup2(1.0f)), dup2(half)), ix = mul2(add2(xn, dup2(1.0f)), dup2(half));
+      float2 v;
+      if constexpr (NI > 0) {
+        // floor by adding 1.5 * 2^23 rounded down: the sum's low bits are the
+        // integer, clamped as they are (the bits of positive floats are ordered)
+        constexpr float kMagic = 12582912.0f;
+        constexpr int kZero = 0x4B400000;  // the bits of kMagic
+        const float2 ry = add2_down(iy, dup2(kMagic)), rx = add2_down(ix, dup2(kMagic));
+        const float2 fy = add2(ry, dup2(-kMagic)), fx = add2(rx, dup2(-kMagic));
+        const float2 w = sub2(ix, fx), ea = sub2(dup2(1.0f), w);
+        const float2 nn = sub2(iy, fy), s = sub2(dup2(1.0f), nn);
+        auto at = [&](float yb, float xb) {
+          const int y0 = min(max(__float_as_int(yb), kZero - kBorder), kZero + N);
+          const int x0 = min(max(__float_as_int(xb), kZero - kBorder), kZero + N);
+          return img + ((y0 - kZero + kBorder) * ILD + (x0 - kZero + kBorder));
+        };
+        const float* a = at(ry.x, rx.x);
+        const float* b = at(ry.y, rx.y);
+        v = mul2(make_float2(a[0], b[0]), mul2(s, ea));
+        v = add2(v, mul2(make_float2(a[1], b[1]), mul2(s, w)));
+        v = add2(v, mul2(make_float2(a[ILD], b[ILD]), mul2(nn, ea)));
+        v = add2(v, mul2(make_float2(a[ILD + 1], b[ILD + 1]), mul2(nn, w)));
+      } else {
+        v.x = sample_bilinear_zero(img, N, iy.x, ix.x);
+        v.y = sample_bilinear_zero(img, N, iy.y, ix.y);
+      }
+      if (P.mask != nullptr) {
+        const float* mk = P.mask + 2 * q * N + j;
+        v = mul2(v, make_float2(__ldg(mk), __ldg(mk + N)));
+      }
+      Z.at(q, j) = v;
+    }
+    __syncthreads();
+    for (int grp = warp; grp < pair_row_groups<N>(); grp += NW) {
+      const PairRows<N> R{Z, grp};
+      line_fft_warp<N, -1>(R, G, s_tw);
+      pair_split_rows<N>(R);
+    }
+    __syncthreads();
+    for (int grp = warp; grp < pair_col_groups<N>(); grp += NW) {
+      line_fft_warp<N, -1>(PairCols<N>{Z, grp * G}, G, s_tw);
+      if (grp == 0) col0_split<N>(Z, s_last);
+    }
+    __syncthreads();
+    // crop, pack, CTF, conjugate: every value is weighted in place (column
+    // nb / 2 in s_last) and squared for the norm, then scaled and written
+    const float* ctf = P.ctf + (size_t)p * nb * H;
+    const int hb = nb / 2;
+    float hi = 0.f, lo = 0.f;
+    for (int r = warp; r < nb; r += NW) {
+      const int i = r < hb ? r : r + N - nb;
+#pragma unroll 2
+      for (int c = lane; c < hb; c += 32) {
+        float2& z = Z.half(i, c);
+        const float2 f = cscale(cconj(z), __ldg(ctf + r * H + c));
+        z = f;
+        add_square(f.x, hi, lo);
+        add_square(f.y, hi, lo);
+      }
+    }
+    for (int r = tid; r < nb; r += NT) {
+      const int i = r < hb ? r : r + N - nb;
+      // cropped: the packed column is the negative frequency -nb / 2, the
+      // conjugate of the stored one, and is conjugated once more here
+      const float2 z = nb == N ? cconj(s_last[i]) : Z.half(i == 0 ? 0 : N - i, hb);
+      const float2 f = cscale(z, __ldg(ctf + r * H + hb));
+      s_last[r] = f;
+      add_square(f.x, hi, lo);
+      add_square(f.y, hi, lo);
+    }
+    const double ss = warp_sum_d((double)hi + (double)lo);
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();
+    if (tid == 0) {  // one thread: FP64 division and square root
+      double total = 0.0;
+      for (int w = 0; w < NW; ++w) total += red[w];
+      red[NW] = 1.0 / sqrt(total);
+    }
+    __syncthreads();
+    const float inv = (float)red[NW];
+    float2* out = P.out + (size_t)job * nb * H;
+    for (int r = warp; r < nb; r += NW) {
+      const int i = r < hb ? r : r + N - nb, rs = r < hb ? r + hb : r - hb;
+#pragma unroll 2
+      for (int c = lane; c <= hb; c += 32) {
+        const int cs = c + H / 2 < H ? c + H / 2 : c + H / 2 - H;
+        out[rs * H + cs] = cscale(c < hb ? Z.half(i, c) : s_last[r], inv);
+      }
+    }
+    __syncthreads();  // the plane, the image and red are free
+  }
+}
+
+template <int N>
+cudaError_t launch_plane(const PrepParams& P, int sm_count, cudaStream_t st) {
+  const size_t smem = (size_t)(pair_elems(N) + 2 * N) * sizeof(float2) + (prep_threads<N>() / 32 + 1) * sizeof(double) +
+                      (size_t)prep_images<N>() * image_elems<N>() * sizeof(float);
+  static size_t set_smem = 0;  // attribute set once, never inside a stream capture
+  if (set_smem < smem) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(prepare_plane<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    set_smem = smem;
+  }
+  // one CTA per SM at 128 and 192 (the plane and the images fill it), two at
+  // 96, five at 64 and as many at 32
+  const long long jobs = (long long)P.n * P.n_psi, most = (long long)sm_count * (N >= 128 ? 1 : (N == 96 ? 2 : 5));
+  prepare_plane<N><<<(int)(jobs < most ? jobs : most), prep_threads<N>(), smem, st>>>(P);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_packed_ctf(cudaStream_t st, const float* dfu, const float* dfv, const float* dfa,
@@ -186,24 +418,35 @@ cudaError_t launch_packed_ctf(cudaStream_t st, const float* dfu, const float* df
   return cudaGetLastError();
 }
 
+// complex elements of one CTA's scratch plane (box 256 only)
 size_t prepare_scratch_elems(int N, int nb) {
-  return (size_t)N * (N / 2 + 1) + (size_t)nb * (nb / 2 + 1);
+  return N == 256 ? (size_t)N * (N / 2 + 1) + (size_t)nb * (nb / 2 + 1) : 0;
 }
 
-size_t prepare_smem_bytes(int N) {
+static size_t prepare_smem_bytes(int N) {
   return (size_t)max(kRowBatch, kColBatch) * N * sizeof(float2) + (kMaxFftLen / 2) * sizeof(float2) +
          40 * sizeof(double);
 }
 
+// grid: CTAs of the box-256 kernel, one scratch plane each (4 per SM)
 cudaError_t launch_prepare_particles(cudaStream_t st, const float* images, int n, int n_psi,
                                      const int* psi_index, const void* psi_tab, const float* mask,
-                                     const float* ctf, float2* out, float2* scratch, int grid,
+                                     const float* ctf, float2* out, float2* scratch, int grid, int sm_count,
                                      const float2* tw, const float2* tw3, int N, int nb) {
   if (n <= 0) return cudaSuccess;
   PrepParams P;
   P.images = images; P.psi_index = psi_index; P.psi_tab = (const float4*)psi_tab; P.mask = mask;
   P.ctf = ctf; P.out = out; P.scratch = scratch; P.scratch_stride = prepare_scratch_elems(N, nb);
   P.tw = tw; P.tw3 = tw3; P.n = n; P.n_psi = n_psi; P.N = N; P.nb = nb;
+  switch (N) {
+    case 32: return launch_plane<32>(P, sm_count, st);
+    case 64: return launch_plane<64>(P, sm_count, st);
+    case 96: return launch_plane<96>(P, sm_count, st);
+    case 128: return launch_plane<128>(P, sm_count, st);
+    case 192: return launch_plane<192>(P, sm_count, st);
+    case 256: break;
+    default: return cudaErrorInvalidValue;
+  }
   const size_t smem = prepare_smem_bytes(N);
   static size_t set_smem = 0;
   if (set_smem < smem) {
