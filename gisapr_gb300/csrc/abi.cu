@@ -26,9 +26,10 @@ cudaError_t launch_splat_bricks(cudaStream_t, const void*, int, const float*, fl
 cudaError_t launch_pad_sinc_shift(cudaStream_t, const float*, float*, int);
 int splat_bin_cap();
 int splat_bin_count(int box);
+int splat_count_elems(int box);
 cudaError_t launch_splat_binned(cudaStream_t, const float*, const float*, int, int, const float*, const double*,
                                 const double*, const float*, float*, float*, int, int, double, double, double, void*,
-                                int*, int*);
+                                int*, int*, int);
 size_t project_scratch_elems(int N, int nb);
 size_t project_smem_bytes(int N, int n_bins);
 cudaError_t launch_project_templates(cudaStream_t, const float2*, const float*, const int*, int,
@@ -402,13 +403,13 @@ static int deposit_common(gisapr_ctx ctx, void* stream, const float* xyz, const 
   rc = ensure(ctx, ctx->atoms, (size_t)(n > 0 ? n : 1) * atom_record_bytes(), "cudaMalloc(atoms)");
   if (rc) return rc;
   const size_t nbricks = (size_t)splat_bin_count(box);
-  rc = ensure(ctx, ctx->bin_counts, nbricks * sizeof(int), "cudaMalloc(brick counts)");
+  rc = ensure(ctx, ctx->bin_counts, splat_count_elems(box) * sizeof(int), "cudaMalloc(brick counts)");
   if (rc) return rc;
   rc = ensure(ctx, ctx->bin_lists, nbricks * splat_bin_cap() * sizeof(int), "cudaMalloc(brick lists)");
   if (rc) return rc;
   GISAPR_CHECK_CUDA(launch_splat_binned(st, xyz, numbers, n, transform, pivot, rot, shift, initial, out, padded,
                                         box, width, apix, rp, kn, ctx->atoms.ptr, (int*)ctx->bin_counts.ptr,
-                                        (int*)ctx->bin_lists.ptr),
+                                        (int*)ctx->bin_lists.ptr, ctx->sm_count),
                     "splat");
   return GISAPR_OK;
 }

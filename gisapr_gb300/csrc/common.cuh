@@ -18,7 +18,9 @@ constexpr int kMaxFftLen = 512;
 // rounded as its scalar form. The FMA pipes do as many operations a cycle as
 // with scalar instructions (measured on GB300: 39.3 against 38.3 T a second),
 // so what a pair saves is issue slots: complex sums in this form took 1% to 3%
-// off the kernels that are made of FFT codelets.
+// off the kernels that are made of FFT codelets. The assembler may still fuse
+// a packed product into the packed sum it feeds (seen in the splat's bits);
+// where both roundings matter the product is scalar (__fmul_rn is never fused).
 GISAPR_DEV unsigned long long f2_bits(float2 a) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
