@@ -16,6 +16,7 @@
 
 #include "../../include/gisapr_gb300.h"
 #include "common.cuh"
+#include "pairplane.cuh"
 
 // ---- launchers defined in the other translation units
 cudaError_t launch_atoms_prepare(cudaStream_t, const float*, const float*, int, int, const float*,
@@ -31,23 +32,14 @@ cudaError_t launch_splat_binned(cudaStream_t, const float*, const float*, int, i
                                 const double*, const float*, float*, float*, int, int, double, double, double, void*,
                                 int*, int*, int);
 size_t project_scratch_elems(int N, int nb);
-size_t project_smem_bytes(int N, int n_bins);
-cudaError_t launch_project_templates(cudaStream_t, const float2*, const float*, const int*, int,
-                                     const int*, const float*, const float*, const int*, const int*,
-                                     const float*, int, const float2*, const float2*, float2*, float2*, int,
-                                     int, int);
-size_t project_smem_bytes_fast(int N, int n_bins, int nb);
-cudaError_t launch_project_templates_fast(cudaStream_t, const float2*, const float*, const int*, int,
-                                          const int*, const float*, const float*, const int*, const int*,
-                                          const float*, int, const float2*, float2*, int, int, int, float2*,
-                                          float2*, int*, unsigned);
 size_t project_blocked_elems(int N);
-size_t project_slice_elems(int N, int n_build);
+size_t project_plane_elems(int N, int n_build);
+cudaError_t launch_project_templates(cudaStream_t, const float2*, const float*, const int*, int, const int*,
+                                     const float*, const float*, const ProjTables&, float2*, float2*, int, int, int,
+                                     float2*, float2*, int*, unsigned);
 cudaError_t launch_project_templates_planes(cudaStream_t, const float2*, const float*, const int*, int,
-                                            const int*, const float*, const float*, const int*, const int*,
-                                            const float*, int, const float2*, const float2*, float2*, float2*,
-                                            int, int, int, float2*, float2*, int);
-size_t project_flat_plane_elems(int N, int n);
+                                            const int*, const float*, const float*, const ProjTables&, float2*,
+                                            float2*, int, int, int, float2*, float2*, int);
 size_t vfft_scratch_elems(int N);
 cudaError_t launch_volume_spectrum_blocked(cudaStream_t, const float*, int, float2*, float2*, const float2*);
 cudaError_t launch_packed_ctf(cudaStream_t, const float*, const float*, const float*, int,
@@ -118,8 +110,10 @@ struct DeviceBuffer {
 
 struct BinTable {
   int* list = nullptr;
+  unsigned short* off = nullptr;  // pair-plane offsets (boxes 32, 64, 128)
   int* ptr = nullptr;
   float* count = nullptr;
+  float2* tw = nullptr;  // twiddles of the warp FFT [N], then exp(-2 pi i t / 2N), t < N
   int n_bins = 0;
 };
 
@@ -239,8 +233,31 @@ int get_bins(gisapr_ctx ctx, int N, BinTable* out) {
   for (int b = 0; b < nb; ++b) ptr[b + 1] += ptr[b];
   std::vector<int> fill(ptr.begin(), ptr.end() - 1);
   for (int i = 0; i < N * HC; ++i) list[fill[bin_of[i]]++] = i;
+  // the same pixels as offsets into the pair plane (the Nyquist column after
+  // the plane), top bit for the columns that stand for themselves only
+  std::vector<unsigned short> off;
+  if (is_pow2(N) && N <= 128) {
+    for (int idx : list) {
+      const int r = idx / HC, kx = idx - r * HC, q = r >> 1, j = kx + (r & 1) * (N / 2);
+      const int o = kx == N / 2 ? pair_elems(N) + r : q * pair_ld(N) + (q >> 2) + j + (j >> 3);
+      off.push_back((unsigned short)(o | (kx == 0 || kx == N / 2 ? 0x8000 : 0)));
+    }
+  }
+  std::vector<float2> tw(2 * N);
+  const double two_pi = 6.283185307179586476925286766559;
+  for (int k = 0; k < N; ++k) {
+    const double a = -two_pi / (double)N, e = (double)((k / (N / 16)) * (k % (N / 16)));
+    tw[k] = make_float2((float)std::cos(a * e), (float)std::sin(a * e));
+    tw[N + k] = make_float2((float)std::cos(0.5 * a * k), (float)std::sin(0.5 * a * k));
+  }
   BinTable t;
   t.n_bins = nb;
+  GISAPR_CHECK_CUDA(cudaMalloc(&t.off, std::max<size_t>(1, off.size()) * sizeof(unsigned short)), "cudaMalloc(bins)");
+  GISAPR_CHECK_CUDA(cudaMemcpy(t.off, off.data(), off.size() * sizeof(unsigned short), cudaMemcpyHostToDevice),
+                    "cudaMemcpy(bins)");
+  GISAPR_CHECK_CUDA(cudaMalloc(&t.tw, tw.size() * sizeof(float2)), "cudaMalloc(bins)");
+  GISAPR_CHECK_CUDA(cudaMemcpy(t.tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice),
+                    "cudaMemcpy(bins)");
   GISAPR_CHECK_CUDA(cudaMalloc(&t.list, list.size() * sizeof(int)), "cudaMalloc(bins)");
   GISAPR_CHECK_CUDA(cudaMalloc(&t.ptr, ptr.size() * sizeof(int)), "cudaMalloc(bins)");
   GISAPR_CHECK_CUDA(cudaMalloc(&t.count, cnt.size() * sizeof(float)), "cudaMalloc(bins)");
@@ -367,7 +384,10 @@ int gisapr_context_destroy(gisapr_ctx ctx) {
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
   for (auto& kv : ctx->fft) { cufftDestroy(kv.second.first); cudaFree(kv.second.second); }
-  for (auto& kv : ctx->bins) { cudaFree(kv.second.list); cudaFree(kv.second.ptr); cudaFree(kv.second.count); }
+  for (auto& kv : ctx->bins) {
+    cudaFree(kv.second.list); cudaFree(kv.second.off); cudaFree(kv.second.ptr); cudaFree(kv.second.count);
+    cudaFree(kv.second.tw);
+  }
   for (auto& kv : ctx->corr) { cudaFree(kv.second.outer); cudaFree(kv.second.col); }
   cudaFree(ctx->atoms.ptr);
   cudaFree(ctx->bin_counts.ptr);
@@ -542,21 +562,19 @@ int gisapr_project_templates(gisapr_ctx ctx, void* stream, const float* spectrum
   BinTable bt;
   rc = get_bins(ctx, box, &bt);
   if (rc) return rc;
+  const ProjTables tables{bt.list, bt.off, bt.ptr, bt.count, bt.n_bins, ctx->tw, ctx->tw3, bt.tw, bt.tw + box};
   if (box <= 128 && is_pow2(box)) {
-    // whole template in shared memory, one CTA per SM
-    const int grid = grid_for(ctx, n_build, 1);
     if (n_build > 65535) return fail(GISAPR_ERR_ARGUMENT, "at most 65535 templates per call");
-    rc = ensure(ctx, ctx->proj_slices, project_slice_elems(box, n_build) * sizeof(float2), "cudaMalloc(planes)");
+    rc = ensure(ctx, ctx->proj_slices, project_plane_elems(box, n_build) * sizeof(float2), "cudaMalloc(planes)");
     if (rc) return rc;
     rc = ensure(ctx, ctx->proj_blocked, project_blocked_elems(box) * sizeof(float2), "cudaMalloc(blocked spectrum)");
     if (rc) return rc;
     rc = status_word(ctx);
     if (rc) return rc;
-    GISAPR_CHECK_CUDA(launch_project_templates_fast((cudaStream_t)stream, (const float2*)spectrum, rot, dirs,
-                                                    n_build, out_slot, mask, fsc, bt.list, bt.ptr, bt.count,
-                                                    bt.n_bins, ctx->tw, (float2*)bank, grid, box, newbox,
-                                                    (float2*)ctx->proj_slices.ptr, (float2*)ctx->proj_blocked.ptr,
-                                                    (int*)ctx->proj_status.ptr, ctx->proj_wait),
+    GISAPR_CHECK_CUDA(launch_project_templates((cudaStream_t)stream, (const float2*)spectrum, rot, dirs, n_build,
+                                               out_slot, mask, fsc, tables, (float2*)bank, nullptr, 0, box, newbox,
+                                               (float2*)ctx->proj_slices.ptr, (float2*)ctx->proj_blocked.ptr,
+                                               (int*)ctx->proj_status.ptr, ctx->proj_wait),
                       "project_templates");
     ctx->blocked_box = box;
     return GISAPR_OK;
@@ -571,13 +589,12 @@ int gisapr_project_templates(gisapr_ctx ctx, void* stream, const float* spectrum
     // the gather and pass A in their own high-occupancy kernel, from the
     // blocked spectrum, at most 4,096 planes (2.2 GB) at a time
     const int chunk = std::min(n_build, kPlaneChunk);
-    rc = ensure(ctx, ctx->proj_slices, project_flat_plane_elems(box, chunk) * sizeof(float2), "cudaMalloc(planes)");
+    rc = ensure(ctx, ctx->proj_slices, project_plane_elems(box, chunk) * sizeof(float2), "cudaMalloc(planes)");
     if (rc) return rc;
     rc = ensure(ctx, ctx->proj_blocked, project_blocked_elems(box) * sizeof(float2), "cudaMalloc(blocked spectrum)");
     if (rc) return rc;
     GISAPR_CHECK_CUDA(launch_project_templates_planes((cudaStream_t)stream, (const float2*)spectrum, rot, dirs,
-                                                      n_build, out_slot, mask, fsc, bt.list, bt.ptr, bt.count,
-                                                      bt.n_bins, ctx->tw, ctx->tw3, (float2*)bank,
+                                                      n_build, out_slot, mask, fsc, tables, (float2*)bank,
                                                       (float2*)ctx->proj_scratch.ptr, grid, box, newbox,
                                                       (float2*)ctx->proj_slices.ptr, (float2*)ctx->proj_blocked.ptr,
                                                       chunk),
@@ -586,9 +603,9 @@ int gisapr_project_templates(gisapr_ctx ctx, void* stream, const float* spectrum
     return GISAPR_OK;
   }
   GISAPR_CHECK_CUDA(launch_project_templates((cudaStream_t)stream, (const float2*)spectrum, rot, dirs, n_build,
-                                             out_slot, mask, fsc, bt.list, bt.ptr, bt.count, bt.n_bins,
-                                             ctx->tw, ctx->tw3, (float2*)bank, (float2*)ctx->proj_scratch.ptr, grid,
-                                             box, newbox),
+                                             out_slot, mask, fsc, tables, (float2*)bank,
+                                             (float2*)ctx->proj_scratch.ptr, grid, box, newbox, nullptr, nullptr,
+                                             nullptr, 0),
                     "project_templates");
   return GISAPR_OK;
 }

@@ -60,6 +60,11 @@ GISAPR_DEV float2 dup2(float a) { return make_float2(a, a); }
 
 GISAPR_DEV float2 cadd(float2 a, float2 b) { return add2(a, b); }
 GISAPR_DEV float2 csub(float2 a, float2 b) { return sub2(a, b); }
+// The same in scalar instructions, for kernels that live on few registers (a
+// packed operand is an aligned pair: the block-wide transforms of box 192 ran 23%
+// slower with pairs).
+GISAPR_DEV float2 cadd_s(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+GISAPR_DEV float2 csub_s(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 GISAPR_DEV float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -104,8 +109,8 @@ GISAPR_DEV void smem_fft_dit(float2* buf, int L, int lines, int line_stride, int
       float2 v = base[(i + half) * elem_stride];
       float2 w = tw[k << tw_shift];
       float2 vt = cmul_sign(v, w, -sign);  // tw is exp(-..): sign=-1 keeps it, +1 conjugates
-      base[i * elem_stride] = cadd(u, vt);
-      base[(i + half) * elem_stride] = csub(u, vt);
+      base[i * elem_stride] = cadd_s(u, vt);
+      base[(i + half) * elem_stride] = csub_s(u, vt);
     }
     __syncthreads();
   }
@@ -160,9 +165,9 @@ GISAPR_DEV void smem_fft(float2* buf, int L, int lines, float sign, const float2
     float2 w1 = tw3[k * scale], w2 = tw3[2 * k * scale];
     if (sign > 0.f) { w1.y = -w1.y; w2.y = -w2.y; }
     const float2 a = base[k], b = cmul(base[L3 + k], w1), c = cmul(base[2 * L3 + k], w2);
-    const float2 s = cadd(b, c), d = csub(b, c);
+    const float2 s = cadd_s(b, c), d = csub_s(b, c);
     const float2 h = make_float2(a.x - 0.5f * s.x, a.y - 0.5f * s.y);
-    base[k] = cadd(a, s);
+    base[k] = cadd_s(a, s);
     base[L3 + k] = make_float2(h.x - s3 * d.y, h.y + s3 * d.x);
     base[2 * L3 + k] = make_float2(h.x + s3 * d.y, h.y - s3 * d.x);
   }
@@ -248,6 +253,19 @@ GISAPR_DEV double block_sum_d(double v, double* scratch) {
   __syncthreads();
   return t;
 }
+
+// Tables of a projector call, kept by the context per box.
+struct ProjTables {
+  const int* bin_list;             // [N (N/2 + 1)] half-plane indices r (N/2 + 1) + k, by radial bin
+  const unsigned short* bin_off;   // the same as offsets into the pair plane, top bit: columns 0 and N/2 (boxes 32, 64, 128)
+  const int* bin_ptr;              // [n_bins + 1]
+  const float* bin_count;          // [n_bins] full-grid counts per bin
+  int n_bins;
+  const float2* tw;                // exp(-2 pi i t / kMaxFftLen)
+  const float2* tw3;               // exp(-2 pi i t / kMaxFftLen3)
+  const float2* tw_n;              // [N] twiddles of the warp FFT, exp(-2 pi i n2 k1 / N) at k1 N/16 + n2
+  const float2* tw_2n;             // [N] exp(-2 pi i t / 2N)
+};
 
 // Status word written by kernels that detect bad input on the device.
 enum GisaprDeviceStatus : int {

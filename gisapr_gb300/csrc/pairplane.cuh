@@ -34,13 +34,26 @@ GISAPR_DEV void dft3(float2& a, float2& b, float2& c) {
   c = csub(h, t);
 }
 
-// exp(DIR * i * k * pi / 6) for k = 0..11
+// exp(DIR * i * k * pi / 6), k = 0..11 known at compile time
 template <int DIR>
 GISAPR_DEV float2 w12(int k) {
   constexpr float kC = 0.86602540378443864676f;
-  const float c[12] = {1.f, kC, 0.5f, 0.f, -0.5f, -kC, -1.f, -kC, -0.5f, 0.f, 0.5f, kC};
-  const float s = c[(k + 9) % 12];
-  return make_float2(c[k % 12], DIR > 0 ? s : -s);
+  float c = 1.f, s = 0.f;
+  switch (k % 12) {
+    case 1: c = kC; s = 0.5f; break;
+    case 2: c = 0.5f; s = kC; break;
+    case 3: c = 0.f; s = 1.f; break;
+    case 4: c = -0.5f; s = kC; break;
+    case 5: c = -kC; s = 0.5f; break;
+    case 6: c = -1.f; break;
+    case 7: c = -kC; s = -0.5f; break;
+    case 8: c = -0.5f; s = -kC; break;
+    case 9: c = 0.f; s = -1.f; break;
+    case 10: c = 0.5f; s = -kC; break;
+    case 11: c = kC; s = -0.5f; break;
+    default: break;
+  }
+  return make_float2(c, DIR > 0 ? s : -s);
 }
 
 // 6 = 2 x 3: n = 3 n1 + n2, k = k1 + 2 k2
@@ -93,25 +106,36 @@ GISAPR_DEV void dft<12, -1>(float2 (&x)[12]) { dft12_impl<-1>(x); }
 template <int N>
 __host__ __device__ constexpr int fft_lines() { return N == 96 ? 4 : (N == 192 ? 2 : 32 / (N / 16)); }
 
-// One warp's in-place four-step transform of ``nlines`` (<= fft_lines<N>())
-// lines, natural order in and out: 16-point codelets over n1, twiddles,
-// N/16-point codelets over n2. ``tw[t]`` = exp(-2 pi i t / N) for t < N (the
-// whole circle of this length, so a twiddle is one load).
-template <int N, int DIR, class Lines>
-GISAPR_DEV void line_fft_warp(const Lines& L, int nlines, const float2* tw) {
-  constexpr int L2 = N / 16, G = fft_lines<N>(), T = (G * 16) / 32;
+// The twiddles between the two steps, exp(-2 pi i n2 k1 / N), in the order the
+// lanes of a warp read them (entry k1 N/16 + n2): one conflict-free load each,
+// where a table by exponent put a warp's eight on two to eight banks.
+template <int N>
+__host__ __device__ constexpr int twiddle_exponent(int entry) { return (entry / (N / 16)) * (entry % (N / 16)); }
+
+// One warp's four-step transform of fft_lines<N>() lines, natural order in
+// and out: 16-point codelets over n1, twiddles, N/16-point codelets over n2.
+// ``load(g, k)`` gives element k of line g, L.at holds the values between the
+// two steps, ``store(g, k, v)`` takes the result. A load may read any element of
+// the warp's lines (all loads come before the first write). LINES: fewer lines.
+// ``tw`` is the table of twiddle_exponent, in shared memory.
+template <int N, int DIR, int LINES = 0, class Lines, class Load, class Store>
+GISAPR_DEV void line_fft_warp(const Lines& L, const float2* tw, const Load& load, const Store& store) {
+  constexpr int L2 = N / 16, G = LINES ? LINES : fft_lines<N>(), T = (G * 16 + 31) / 32;
   const int lane = threadIdx.x & 31;
   {
     const int g = lane / L2, n2 = lane % L2;
-    if (g < nlines) {
-      float2 x[16];
+    float2 x[16];
+    if (G * L2 == 32 || g < G) {
 #pragma unroll
-      for (int n1 = 0; n1 < 16; ++n1) x[n1] = L.at(g, L2 * n1 + n2);
+      for (int n1 = 0; n1 < 16; ++n1) x[n1] = load(g, L2 * n1 + n2);
       dft<16, DIR>(x);
+    }
+    __syncwarp();
+    if (G * L2 == 32 || g < G) {
       L.at(g, n2) = x[0];
 #pragma unroll
       for (int k1 = 1; k1 < 16; ++k1) {
-        const float2 w = tw[n2 * k1];
+        const float2 w = tw[k1 * L2 + n2];
         L.at(g, L2 * k1 + n2) = cmul(x[k1], DIR < 0 ? w : cconj(w));
       }
     }
@@ -121,7 +145,7 @@ GISAPR_DEV void line_fft_warp(const Lines& L, int nlines, const float2* tw) {
 #pragma unroll
   for (int t = 0; t < T; ++t) {
     const int task = lane + 32 * t, g = task / 16, k1 = task % 16;
-    if (g < nlines) {
+    if (G * 16 % 32 == 0 || g < G) {
 #pragma unroll
       for (int n2 = 0; n2 < L2; ++n2) y[t][n2] = L.at(g, L2 * k1 + n2);
       dft<L2, DIR>(y[t]);
@@ -131,15 +155,36 @@ GISAPR_DEV void line_fft_warp(const Lines& L, int nlines, const float2* tw) {
 #pragma unroll
   for (int t = 0; t < T; ++t) {
     const int task = lane + 32 * t, g = task / 16, k1 = task % 16;
-    if (g < nlines) {
+    if (G * 16 % 32 == 0 || g < G) {
 #pragma unroll
-      for (int k2 = 0; k2 < L2; ++k2) L.at(g, k1 + 16 * k2) = y[t][k2];
+      for (int k2 = 0; k2 < L2; ++k2) store(g, k1 + 16 * k2, y[t][k2]);
     }
   }
   __syncwarp();
 }
 
-// entry t of the twiddle table of length N, from the context's two tables
+// The same in place.
+template <int N, int DIR, class Lines>
+GISAPR_DEV void line_fft_warp(const Lines& L, const float2* tw) {
+  line_fft_warp<N, DIR>(L, tw, [&](int g, int k) { return L.at(g, k); },
+                        [&](int g, int k, float2 v) { L.at(g, k) = v; });
+}
+
+// Staging lines of one warp (powers of two): element k of a line at
+// k ^ (its row of 16), line stride N + N/16 and four slots more every two lines:
+// the loads and stores of both steps, and the slice gather's, fall on distinct
+// banks at N = 128.
+__host__ __device__ constexpr int stage_ld(int N) { return N + N / 16; }
+__host__ __device__ constexpr int stage_elems(int N, int lines) { return lines * stage_ld(N) + 2 * lines; }
+template <int N>
+struct StagedLines {
+  float2* p;
+  GISAPR_DEV static int slot(int k) { return k ^ ((k >> 4) & (N / 16 - 1)); }
+  GISAPR_DEV float2* line(int g) const { return p + g * stage_ld(N) + (g >> 1) * 4; }
+  GISAPR_DEV float2& at(int g, int k) const { return line(g)[slot(k)]; }
+};
+
+// exp(-2 pi i t / N), from the context's two tables
 template <int N>
 GISAPR_DEV float2 twiddle_of(const float2* __restrict__ tw, const float2* __restrict__ tw3, int t) {
   if constexpr ((N & (N - 1)) == 0) return tw_full<-1>(tw, t, N);

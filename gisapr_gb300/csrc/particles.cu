@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(prep_threads<N>(), N <= 64 ? 4 : (N == 96 ? 2 
   const PairPlane<N> Z{plane};
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nb = P.nb, H = nb / 2 + 1;
-  for (int t = tid; t < N; t += NT) s_tw[t] = twiddle_of<N>(P.tw, P.tw3, t);
+  for (int t = tid; t < N; t += NT) s_tw[t] = twiddle_of<N>(P.tw, P.tw3, twiddle_exponent<N>(t));
   for (int t = tid; t < NI * IEL; t += NT) s_img[t] = 0.f;  // the border stays zero
   const long long jobs = (long long)P.n * P.n_psi;
   const int j0 = (int)(jobs * blockIdx.x / gridDim.x), j1 = (int)(jobs * (blockIdx.x + 1) / gridDim.x);
@@ -329,12 +329,12 @@ __global__ void __launch_bounds__(prep_threads<N>(), N <= 64 ? 4 : (N == 96 ? 2 
     __syncthreads();
     for (int grp = warp; grp < pair_row_groups<N>(); grp += NW) {
       const PairRows<N> R{Z, grp};
-      line_fft_warp<N, -1>(R, G, s_tw);
+      line_fft_warp<N, -1>(R, s_tw);
       pair_split_rows<N>(R);
     }
     __syncthreads();
     for (int grp = warp; grp < pair_col_groups<N>(); grp += NW) {
-      line_fft_warp<N, -1>(PairCols<N>{Z, grp * G}, G, s_tw);
+      line_fft_warp<N, -1>(PairCols<N>{Z, grp * G}, s_tw);
       if (grp == 0) col0_split<N>(Z, s_last);
     }
     __syncthreads();
