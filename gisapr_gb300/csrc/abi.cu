@@ -62,12 +62,11 @@ cudaError_t launch_restraint_edt(cudaStream_t, const float*, float, unsigned cha
 cudaError_t launch_restraint_init(cudaStream_t, int*, int);
 cudaError_t launch_restraint_reduce(cudaStream_t, float*, const unsigned char*, const int*, int, const int*,
                                     const int*, float, int*, int);
-cudaError_t launch_ingest_load(cudaStream_t, const float*, int, int, int, const int*, int, int, double2*, int);
-cudaError_t launch_ingest_spectrum_divide(cudaStream_t, double2*, int, int, const int*, const int*, const double*,
-                                          int);
-cudaError_t launch_ingest_normalize(cudaStream_t, double2*, int, int, int, double);
-cudaError_t launch_ingest_scale_mask(cudaStream_t, double2*, int, int, const double*, double, int, int);
-cudaError_t launch_ingest_store(cudaStream_t, const double2*, int, int, double, float*, int);
+cudaError_t launch_ingest_load(cudaStream_t, const float*, int, int, int, const int*, int, int, double*, int, int);
+cudaError_t launch_ingest_spectrum(cudaStream_t, double2*, int, int, int, const int*, const int*, const double*, int,
+                                   int, const double*);
+cudaError_t launch_ingest_normalize(cudaStream_t, double*, int, int, int, int);
+cudaError_t launch_ingest_store(cudaStream_t, const double*, int, int, int, int, float*, int);
 int correlate_tc_max_psi();
 int correlate_tc_max_n();
 size_t correlate_tc_smem_bytes(int n, int crop, int split, int sa, int sb);
@@ -123,6 +122,16 @@ struct CorrTables {
   float2* row = nullptr;    // [n] exp(+2 pi i t / n)
 };
 
+// Transforms of the particle preparation for one (rows, columns, images).
+struct IngestPlan {
+  int ch = 0, cw = 0, n = 0;
+  cufftHandle forward = 0, inverse = 0;
+  cudaEvent_t done = nullptr;    // the last call's transforms have run
+  cudaStream_t stream = nullptr; // and where
+  unsigned long long used = 0;   // for the choice of the one to give up
+};
+constexpr int kIngestPlans = 4;
+
 }  // namespace
 
 // Lets the other translation units of the library report errors through
@@ -135,6 +144,8 @@ struct gisapr_context {
   float2* tw3 = nullptr;  // exp(-2 pi i t / kMaxFftLen3), t < kMaxFftLen3 (lengths 3 * 2^k)
   std::map<int, std::pair<cufftHandle, float*>> fft;  // box -> (R2C plan, padded input)
   std::map<int, BinTable> bins;                        // N -> radial bins
+  std::vector<IngestPlan> ingest;                      // at most kIngestPlans
+  unsigned long long ingest_calls = 0;
   std::map<std::pair<int, int>, CorrTables> corr;      // (n, crop) -> twiddles
   DeviceBuffer atoms, bin_counts, bin_lists, proj_scratch, prep_scratch, proj_slices, proj_blocked, vfft_scratch;
   DeviceBuffer proj_status;        // int: set to 1 by a projector plane wait that ran out
@@ -272,6 +283,54 @@ int get_bins(gisapr_ctx ctx, int N, BinTable* out) {
   return GISAPR_OK;
 }
 
+// The plans of ch x cw x n, kept with the context: making them took 0.4 ms of a
+// call and destroying them a wait for the stream. A fifth shape replaces the one
+// used longest ago. A plan's work area is one per plan, so a call on another
+// stream waits for the last one.
+int get_ingest_plan(gisapr_ctx ctx, int ch, int cw, int n, cudaStream_t st, IngestPlan** out) {
+  IngestPlan* p = nullptr;
+  for (auto& e : ctx->ingest)
+    if (e.ch == ch && e.cw == cw && e.n == n) p = &e;
+  if (p == nullptr) {
+    if ((int)ctx->ingest.size() == kIngestPlans) {
+      auto old = std::min_element(ctx->ingest.begin(), ctx->ingest.end(),
+                                  [](const IngestPlan& a, const IngestPlan& b) { return a.used < b.used; });
+      cudaEventSynchronize(old->done);
+      cufftDestroy(old->forward);
+      cufftDestroy(old->inverse);
+      cudaEventDestroy(old->done);
+      ctx->ingest.erase(old);
+    }
+    IngestPlan e;
+    e.ch = ch; e.cw = cw; e.n = n; e.stream = st;
+    int dims[2] = {ch, cw}, real[2] = {ch, 2 * (cw / 2 + 1)}, half[2] = {ch, cw / 2 + 1};
+    const int dr = real[0] * real[1], dh = half[0] * half[1];
+    cufftResult r = cufftPlanMany(&e.forward, 2, dims, real, 1, dr, half, 1, dh, CUFFT_D2Z, n);
+    if (r != CUFFT_SUCCESS)
+      return fail(GISAPR_ERR_CUFFT, "cufftPlanMany(D2Z) failed with code " + std::to_string((int)r));
+    r = cufftPlanMany(&e.inverse, 2, dims, half, 1, dh, real, 1, dr, CUFFT_Z2D, n);
+    if (r != CUFFT_SUCCESS) {
+      cufftDestroy(e.forward);
+      return fail(GISAPR_ERR_CUFFT, "cufftPlanMany(Z2D) failed with code " + std::to_string((int)r));
+    }
+    const cudaError_t err = cudaEventCreateWithFlags(&e.done, cudaEventDisableTiming);
+    if (err != cudaSuccess) {
+      cufftDestroy(e.forward);
+      cufftDestroy(e.inverse);
+      return cuda_fail(err, "cudaEventCreate(ingest)");
+    }
+    ctx->ingest.push_back(e);
+    p = &ctx->ingest.back();
+  }
+  if (p->stream != st) GISAPR_CHECK_CUDA(cudaStreamWaitEvent(st, p->done, 0), "cudaStreamWaitEvent(ingest)");
+  p->stream = st;
+  p->used = ++ctx->ingest_calls;
+  cufftSetStream(p->forward, st);
+  cufftSetStream(p->inverse, st);
+  *out = p;
+  return GISAPR_OK;
+}
+
 int get_corr_tables(gisapr_ctx ctx, int n, int crop, CorrTables* out) {
   auto key = std::make_pair(n, crop);
   auto it = ctx->corr.find(key);
@@ -384,6 +443,7 @@ int gisapr_context_destroy(gisapr_ctx ctx) {
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
   for (auto& kv : ctx->fft) { cufftDestroy(kv.second.first); cudaFree(kv.second.second); }
+  for (auto& p : ctx->ingest) { cufftDestroy(p.forward); cufftDestroy(p.inverse); cudaEventDestroy(p.done); }
   for (auto& kv : ctx->bins) {
     cudaFree(kv.second.list); cudaFree(kv.second.off); cudaFree(kv.second.ptr); cudaFree(kv.second.count);
     cudaFree(kv.second.tw);
@@ -912,54 +972,30 @@ int gisapr_ingest_stack(gisapr_ctx ctx, void* stream, const float* images, int n
   int rc = set_device(ctx);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  const int pixels = ch * cw;
-  double2* wk = (double2*)work;
-  GISAPR_CHECK_CUDA(launch_ingest_load(st, images, n, h, w, shifts, ch, cw, wk, ctx->sm_count), "ingest_load");
-  cufftHandle plan = 0;
+  // with transforms, real rows in the padded layout of the in-place D2Z, which
+  // the caller's ch * cw complex values always hold
+  const int ld = (flags & 5) ? 2 * (cw / 2 + 1) : cw;
+  IngestPlan* plan = nullptr;
   if (flags & 5) {
-    int dims[2] = {ch, cw};
-    cufftResult r = cufftPlanMany(&plan, 2, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_Z2Z, n);
-    if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftPlanMany(Z2Z) failed with code " + std::to_string((int)r));
-    cufftSetStream(plan, st);
+    rc = get_ingest_plan(ctx, ch, cw, n, st, &plan);
+    if (rc) return rc;
   }
-  auto run = [&]() -> int {
-    const double inv = 1.0 / (double)pixels;
-    double scale = 1.0;  // pending factor of the values in work
-    if (flags & 1) {
-      cufftResult r = cufftExecZ2Z(plan, (cufftDoubleComplex*)wk, (cufftDoubleComplex*)wk, CUFFT_FORWARD);
-      if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecZ2Z failed");
-      GISAPR_CHECK_CUDA(launch_ingest_spectrum_divide(st, wk, n, pixels, bin_ptr, bin_pix, bin_count, n_bins),
-                        "ingest_spectrum_divide");
-      r = cufftExecZ2Z(plan, (cufftDoubleComplex*)wk, (cufftDoubleComplex*)wk, CUFFT_INVERSE);
-      if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecZ2Z failed");
-      scale = inv;
-    }
-    if (flags & 2) {
-      GISAPR_CHECK_CUDA(launch_ingest_normalize(st, wk, n, ch, cw, scale), "ingest_normalize");
-      scale = 1.0;
-    }
-    if (flags & 4) {
-      if (scale != 1.0)  // the real image of the preceding inverse transform
-        GISAPR_CHECK_CUDA(launch_ingest_scale_mask(st, wk, n, pixels, nullptr, scale, 1, ctx->sm_count),
-                          "ingest_scale");
-      cufftResult r = cufftExecZ2Z(plan, (cufftDoubleComplex*)wk, (cufftDoubleComplex*)wk, CUFFT_FORWARD);
-      if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecZ2Z failed");
-      GISAPR_CHECK_CUDA(launch_ingest_scale_mask(st, wk, n, pixels, highpass_mask, 1.0, 0, ctx->sm_count),
-                        "ingest_mask");
-      r = cufftExecZ2Z(plan, (cufftDoubleComplex*)wk, (cufftDoubleComplex*)wk, CUFFT_INVERSE);
-      if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecZ2Z failed");
-      scale = inv;
-    }
-    GISAPR_CHECK_CUDA(launch_ingest_store(st, wk, n, pixels, scale, out, ctx->sm_count), "ingest_store");
-    return GISAPR_OK;
-  };
-  rc = run();
-  if (plan) {
-    // the plan's work area may be in use until the stream reaches this point
-    cudaStreamSynchronize(st);
-    cufftDestroy(plan);
+  GISAPR_CHECK_CUDA(launch_ingest_load(st, images, n, h, w, shifts, ch, cw, work, ld, ctx->sm_count), "ingest_load");
+  if (flags & 5) {
+    cufftResult r = cufftExecD2Z(plan->forward, (cufftDoubleReal*)work, (cufftDoubleComplex*)work);
+    if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecD2Z failed");
+    GISAPR_CHECK_CUDA(launch_ingest_spectrum(st, (double2*)work, n, ch, cw, (flags & 1) ? bin_ptr : nullptr, bin_pix,
+                                             bin_count, n_bins, (flags & 2) ? 1 : 0,
+                                             (flags & 4) ? highpass_mask : nullptr),
+                      "ingest_spectrum");
+    r = cufftExecZ2D(plan->inverse, (cufftDoubleComplex*)work, (cufftDoubleReal*)work);
+    if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecZ2D failed");
+    GISAPR_CHECK_CUDA(cudaEventRecord(plan->done, st), "cudaEventRecord(ingest)");
+  } else if (flags & 2) {
+    GISAPR_CHECK_CUDA(launch_ingest_normalize(st, work, n, ch, cw, ld), "ingest_normalize");
   }
-  return rc;
+  GISAPR_CHECK_CUDA(launch_ingest_store(st, work, n, ch, cw, ld, out, ctx->sm_count), "ingest_store");
+  return GISAPR_OK;
 }
 
 int gisapr_restraint_edt(gisapr_ctx ctx, void* stream, const float* density, int box, float threshold,

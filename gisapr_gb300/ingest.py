@@ -6,8 +6,8 @@ whitens (divides the spectrum by its radial mean amplitude, then removes a
 least-squares plane and normalises to zero mean and unit sigma) and
 high-pass filters it, writing new stacks and a new STAR (v5:135-277). Here a
 whole chunk of particles goes through one batched float64 pipeline on the
-device (csrc/ingest.cu: load + crop, cuFFT Z2Z, radial-bin divide,
-normalise, mask multiply); the functions of the reference's module keep
+device (csrc/ingest.cu: load + crop, cuFFT D2Z, radial-bin divide, plane
+removal, normalisation and mask in the half spectrum, Z2D); the functions of the reference's module keep
 their names and take one image or a stack:
 
 * ``translation_twoD_image(image, trans_X, trans_Y)`` (v5:9-29) -- host;

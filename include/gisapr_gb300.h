@@ -345,7 +345,10 @@ int gisapr_score_sum_batch(void* stream, const int* local_ptr, const float* peak
  * indices of the unshifted transform grid per bin round(centred radius),
  * bin_count = pixels per bin), 2 = least-squares plane removal and mean/sigma
  * normalisation (normalize), 4 = high-pass by highpass_mask (ch*cw doubles,
- * unshifted order). work: n*ch*cw*2 doubles; out: n float32 ch x cw images.
+ * unshifted order, radial). Bins and mask depend on the centred radius alone:
+ * the steps run in the half spectrum of real images. The context keeps the
+ * transform plans of the last four (ch, cw, n).
+ * work: n*ch*cw*2 doubles; out: n float32 ch x cw images.
  * Every pointer but shifts is device memory.
  */
 int gisapr_ingest_stack(gisapr_ctx ctx, void* stream, const float* images, int n, int h, int w, const int* shifts,
