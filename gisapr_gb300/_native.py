@@ -56,6 +56,7 @@ SIGNATURES = {
     "gisapr_ingest_stack": [_p, _p, _p, _i, _i, _i, _p, _i, _i, _i, _p, _p, _p, _i, _p, _p, _p],
     "gisapr_restraint_init": [_p, _p, _i],
     "gisapr_restraint_eval": [_p, _p, _p, _p, _p, _i, _p, _f, _p],
+    "gisapr_restraint_poses": [_p, _p, _p, _p, _i, _i, _p, _p, _p, _i, _i, _d, _d, _d, _f, _p],
 }
 
 # functions that return something other than an int status (gisapr_project_launches

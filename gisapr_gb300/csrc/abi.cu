@@ -60,6 +60,10 @@ cudaError_t launch_score_sum(cudaStream_t, const int*, const float*, int, double
 size_t edt_smem_bytes(int box);
 cudaError_t launch_restraint_edt(cudaStream_t, const float*, float, unsigned char*, int*, int*, int);
 cudaError_t launch_restraint_init(cudaStream_t, int*, int);
+int restraint_max_poses();
+cudaError_t launch_restraint_poses(cudaStream_t, const float*, const float*, int, int, const int*, const int*,
+                                   const unsigned char*, const int*, float, int*, int, int, double, double, double,
+                                   void*, int*, int*, int);
 cudaError_t launch_restraint_reduce(cudaStream_t, float*, const unsigned char*, const int*, int, const int*,
                                     const int*, float, int*, int);
 cudaError_t launch_ingest_load(cudaStream_t, const float*, int, int, int, const int*, int, int, double*, int, int);
@@ -1031,6 +1035,63 @@ int gisapr_restraint_eval(gisapr_ctx ctx, void* stream, float* volume, const uns
   GISAPR_CHECK_CUDA(launch_restraint_reduce((cudaStream_t)stream, volume, mask, d2, box, bounds, bounds + 3,
                                             threshold, out, ctx->sm_count),
                     "restraint_reduce");
+  return GISAPR_OK;
+}
+
+int gisapr_restraint_poses(gisapr_ctx ctx, void* stream, const float* xyz, const float* numbers, int n_atoms,
+                           int n_poses, const int* bounds, const unsigned char* mask, const int* d2, int box, int width,
+                           double apix, double rp, double kn, float threshold, int* out) {
+  if (!ctx) return fail(GISAPR_ERR_ARGUMENT, "context is NULL");
+  if (n_atoms < 0 || n_poses < 0) return fail(GISAPR_ERR_ARGUMENT, "n_atoms < 0 or n_poses < 0");
+  if (n_poses > 0 && (!bounds || !mask || !d2 || !out || (n_atoms > 0 && (!xyz || !numbers))))
+    return fail(GISAPR_ERR_ARGUMENT, "a required pointer is NULL");
+  if (box < 1 || box > 1024) return fail(GISAPR_ERR_ARGUMENT, "box must be in [1, 1024]");
+  if (width < 3) return fail(GISAPR_ERR_ARGUMENT, "width must be >= 3 (insufficient sampling)");
+  if (!(apix > 0.0) || !std::isfinite(apix) || !std::isfinite(rp) || !std::isfinite(kn))
+    return fail(GISAPR_ERR_ARGUMENT, "apix, rp and kn must be positive and finite");
+  for (int c = 0; c < n_poses; ++c)
+    for (int a = 0; a < 3; ++a)
+      if (bounds[6 * c + a] < 0 || bounds[6 * c + 3 + a] > box || bounds[6 * c + a] > bounds[6 * c + 3 + a])
+        return fail(GISAPR_ERR_ARGUMENT, "bounds must satisfy 0 <= lo <= hi <= box on every axis");
+  int rc = set_device(ctx);
+  if (rc) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (n_poses > 0) GISAPR_CHECK_CUDA(launch_restraint_init(st, out, n_poses), "restraint_init");
+  if (n_atoms == 0) return GISAPR_OK;
+  // Poses share a launch as far as their bricks fit the box's arrays and their
+  // records 200 MB.
+  const int capacity = splat_bin_count(box);
+  const int most = std::max(1, std::min(restraint_max_poses(), (1 << 22) / n_atoms));
+  for (int c0 = 0; c0 < n_poses;) {
+    std::vector<int> lo, num;
+    int count = 0;
+    long long bricks = 0;
+    for (; c0 + count < n_poses && count < most; ++count) {
+      const int* b = bounds + 6 * (c0 + count);  // z0, y0, x0, z1, y1, x1
+      int l[3], m[3];
+      for (int a = 0; a < 3; ++a) {
+        l[a] = b[2 - a] / 8;
+        m[a] = b[5 - a] > b[2 - a] ? (b[5 - a] + 7) / 8 - l[a] : 0;
+      }
+      const long long mine = (long long)m[0] * m[1] * m[2];
+      if (bricks + mine > capacity) break;  // one pose always fits
+      bricks += mine;
+      lo.insert(lo.end(), l, l + 3);
+      num.insert(num.end(), m, m + 3);
+    }
+    rc = ensure(ctx, ctx->atoms, (size_t)count * n_atoms * atom_record_bytes(), "cudaMalloc(atoms)");
+    if (rc) return rc;
+    rc = ensure(ctx, ctx->bin_counts, splat_count_elems(box) * sizeof(int), "cudaMalloc(brick counts)");
+    if (rc) return rc;
+    rc = ensure(ctx, ctx->bin_lists, (size_t)capacity * splat_bin_cap() * sizeof(int), "cudaMalloc(brick lists)");
+    if (rc) return rc;
+    GISAPR_CHECK_CUDA(launch_restraint_poses(st, xyz + (size_t)c0 * n_atoms * 3, numbers, n_atoms, count, lo.data(),
+                                             num.data(), mask, d2, threshold, out + 3 * c0, box, width, apix, rp, kn,
+                                             ctx->atoms.ptr, (int*)ctx->bin_counts.ptr, (int*)ctx->bin_lists.ptr,
+                                             ctx->sm_count),
+                      "restraint_poses");
+    c0 += count;
+  }
   return GISAPR_OK;
 }
 

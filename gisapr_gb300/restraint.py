@@ -8,15 +8,15 @@ main body (every atom not in the chain) is splatted once at ``apix`` with
 resolution 2*apix, thresholded into a mask, and its exact distance
 transform is kept on the device as integer squared voxel distances. A pose
 moves the chain with the reference's float32 row-vector rotation about its
-mean (v8:33-45, on the host, as the reference computes it), the moved chain
-is splatted onto an all-zero scratch volume, and one reduction over the
-chain's bounding box counts overlap voxels and takes the minimum squared
-distance (the scratch is zeroed as it is read). ``evaluate_many`` scores a
-list of poses with one upload of every pose's coordinates, one splat and
-one reduction launch per pose, and one read-back of all results.
+mean (v8:33-45, on the host, as the reference computes it), and the moved
+chain's density is met with mask and distance transform voxel by voxel as it
+is computed: overlap voxels are counted and the minimum squared distance
+taken, with no volume in between. ``evaluate_many`` scores a list of poses
+with one upload of every pose's coordinates, the splat of up to 32 poses in
+one launch, and one read-back of all results.
 
-The kernels are in csrc/restraint.cu; the densities use the same splat as
-the scoring path. There is no CPU path.
+The kernels are in csrc/splat.cu and csrc/restraint.cu; the densities use the
+same splat as the scoring path. There is no CPU path.
 """
 from __future__ import annotations
 
@@ -118,6 +118,36 @@ class GeometryRestraint:
         hi = np.maximum(hi, lo)
         return np.ascontiguousarray(np.concatenate([lo, hi]), dtype=np.int32)
 
+    def _reach(self, lo, hi) -> np.ndarray:
+        """Half-open (z, y, x) voxel boxes [k][6] that hold every voxel the splat
+        of atoms between the corners ``lo`` and ``hi`` [k][3] (Angstrom) can touch."""
+        n, w = self.boxsize, self.width
+        lo = np.floor(lo / self.apix + n // 2 - w) - 2
+        hi = np.ceil(hi / self.apix + n // 2 + w) + 3
+        known = np.isfinite(lo + hi).all(axis=1, keepdims=True)  # an atom at no finite place is not splatted
+        lo = np.clip(np.where(known, lo, 0), 0, n).astype(np.int32)[:, ::-1]
+        hi = np.clip(np.where(known, hi, 0), 0, n).astype(np.int32)[:, ::-1]
+        return np.ascontiguousarray(np.concatenate([lo, np.maximum(hi, lo)], axis=1))
+
+    def _moved(self, poses, pivot):
+        """The chain at every pose [k][n][3], as ``rotate_coords_rotvec`` gives it,
+        and the corners of a box around each: the chain's sphere about the
+        rotation centre, with room for the float32 rounding."""
+        from scipy.spatial.transform import Rotation
+        coords = self.chain_coords
+        center = np.mean(coords, axis=0) if pivot is None else np.asarray(pivot, dtype=np.float32)
+        if center.shape != (3,) or not np.isfinite(center).all():
+            raise ValueError("pivot must contain three finite coordinates in Angstrom")
+        omega = poses[:, :3].astype(np.float32)
+        matrices = Rotation.from_rotvec(np.deg2rad(omega)).as_matrix().astype(np.float32, copy=False)
+        shifts = poses[:, 3:].astype(np.float32)
+        arms = coords - center
+        moved = ((arms @ matrices) + center + shifts[:, None, :]).astype(np.float32, copy=False)
+        middle = center.astype(np.float64) + shifts.astype(np.float64)
+        arm = np.sqrt(np.square(arms, dtype=np.float64).sum(axis=1).max())
+        arm = arm * (1 + 1e-4) + 1e-6 * (np.abs(middle) + np.abs(center))
+        return moved, middle - arm, middle + arm
+
     def _empty_distance(self) -> float:
         # No chain voxel above the threshold: the reference's distance
         # transform then measures to the implicit point (-1, 0, 0) (v8:119-126).
@@ -138,31 +168,25 @@ class GeometryRestraint:
             raise ValueError("pose must contain six finite rotation/translation values")
         if not self.has_mainbody:
             return [(0, 0.0)] * len(poses)
-        k, n_atoms = len(poses), len(self.chain_coords)
-        moved = np.stack([rotate_coords_rotvec(self.chain_coords, *p, pivot=pivot) for p in poses]) \
-            if n_atoms else np.zeros((k, 0, 3), np.float32)
-        bounds = [self._bounds(m) for m in moved]
+        if not len(poses):
+            raise ValueError("need at least one pose")
+        moved, lo, hi = self._moved(poses, pivot)
+        reach = self._reach(lo, hi)
+        k, n_atoms = moved.shape[:2]
         dev = self.device
-        xyz_host = torch.from_numpy(np.ascontiguousarray(moved, dtype=np.float32)).pin_memory()
+        xyz_host = torch.from_numpy(np.ascontiguousarray(moved)).pin_memory()
         xyz = xyz_host.to(dev, non_blocking=True)
         out = torch.empty((k, 3), dtype=torch.int32, device=dev)
         ctx = nat.Context.for_device(dev).handle
         st = nat.stream_of(dev)
         n = self.boxsize
-        nat.call("gisapr_restraint_init", st, nat.ptr(out), k)
-        try:
-            for c in range(k):
-                if n_atoms:
-                    nat.call("gisapr_deposit", ctx, st, nat.c_ptr_offset(xyz, c * n_atoms * 12),
-                             nat.ptr(self.chain_numbers), n_atoms, nat.ptr(self._volume), n, self.width,
-                             self.apix, self.rp, self.kn)
-                nat.call("gisapr_restraint_eval", ctx, st, nat.ptr(self._volume), nat.ptr(self.mainbody_mask),
-                         nat.ptr(self.mainbody_d2), n, bounds[c].ctypes.data, self.threshold,
-                         nat.c_ptr_offset(out, c * 12))
-            res = out.cpu().numpy()
-        except BaseException:
-            self._volume.zero_()
-            raise
+        if self.threshold < 0.0:  # voxels that no atom reaches count as well: a volume per pose
+            self._evaluate_volumes(ctx, st, xyz, [self._bounds(m) for m in moved], out)
+        else:
+            nat.call("gisapr_restraint_poses", ctx, st, nat.ptr(xyz), nat.ptr(self.chain_numbers), n_atoms, k,
+                     reach.ctypes.data, nat.ptr(self.mainbody_mask), nat.ptr(self.mainbody_d2), n, self.width,
+                     self.apix, self.rp, self.kn, self.threshold, nat.ptr(out))
+        res = out.cpu().numpy()
         results = []
         for count, d2, any_voxel in res:
             if count:
@@ -172,6 +196,22 @@ class GeometryRestraint:
             else:
                 results.append((0, self._empty_distance()))
         return results
+
+    def _evaluate_volumes(self, ctx, st, xyz, bounds, out) -> None:
+        k, n_atoms = xyz.shape[:2]
+        n = self.boxsize
+        nat.call("gisapr_restraint_init", st, nat.ptr(out), k)
+        try:
+            for c in range(k):
+                nat.call("gisapr_deposit", ctx, st, nat.c_ptr_offset(xyz, c * n_atoms * 12),
+                         nat.ptr(self.chain_numbers), n_atoms, nat.ptr(self._volume), n, self.width, self.apix,
+                         self.rp, self.kn)
+                nat.call("gisapr_restraint_eval", ctx, st, nat.ptr(self._volume), nat.ptr(self.mainbody_mask),
+                         nat.ptr(self.mainbody_d2), n, bounds[c].ctypes.data, self.threshold,
+                         nat.c_ptr_offset(out, c * 12))
+        except BaseException:
+            self._volume.zero_()
+            raise
 
 
 def create_BOUNDARY_CHECK_parser():

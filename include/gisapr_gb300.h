@@ -381,6 +381,18 @@ int gisapr_restraint_init(void* stream, int* out, int n);
 int gisapr_restraint_eval(gisapr_ctx ctx, void* stream, float* volume, const unsigned char* mask, const int* d2,
                           int box, const int* bounds, float threshold, int* out);
 
+/*
+ * The candidates of one call together (v8:96-126): the moved chain of every
+ * pose, xyz [n_poses][n_atoms][3] (device), splatted onto zeros as
+ * gisapr_deposit does, and reduced against mask and d2 as gisapr_restraint_eval
+ * does into out [n_poses][3], which is set here. bounds: per pose {z0, y0, x0,
+ * z1, y1, x1} (host memory), half-open, holding every voxel the pose's atoms
+ * reach inside the box.
+ */
+int gisapr_restraint_poses(gisapr_ctx ctx, void* stream, const float* xyz, const float* numbers, int n_atoms,
+                           int n_poses, const int* bounds, const unsigned char* mask, const int* d2, int box, int width,
+                           double apix, double rp, double kn, float threshold, int* out);
+
 #ifdef __cplusplus
 }
 #endif
