@@ -54,6 +54,9 @@ size_t correlate_smem_bytes(int n, int n_psi, int crop, int cluster);
 cudaError_t launch_correlate_plain(cudaStream_t, const float2*, const float2*, const int*,
                                    const int*, int, int, int, int, const float2*, const float2*,
                                    float*, int*, int*, int, long long, int, int, const unsigned char*);
+cudaError_t launch_correlate_rows(cudaStream_t, const float2*, const float2*, const int*,
+                                   const int*, int, int, int, int, const float2*, const float2*,
+                                   float*, int*, int*, int, long long, int, int, const unsigned char*, int, bool*);
 cudaError_t launch_particle_results(cudaStream_t, const int*, const float*, const int*, const int*,
                                     int, int, int*, int*, float*, int*, int*, float*, int, const unsigned char*);
 cudaError_t launch_score_sum(cudaStream_t, const int*, const float*, int, double*, int, const unsigned char*);
@@ -737,6 +740,12 @@ int gisapr_correlate_batch_subset(gisapr_ctx ctx, void* stream, const float* ban
   rc = get_corr_tables(ctx, n, crop, &t);
   if (rc) return rc;
   if (nnz < 0) return fail(GISAPR_ERR_ARGUMENT, "nnz < 0");
+  bool taken;
+  GISAPR_CHECK_CUDA(launch_correlate_rows((cudaStream_t)stream, (const float2*)bank, (const float2*)stack,
+                                          local_ptr, local_idx, n_particles, n_psi, n, crop, t.outer, t.col,
+                                          out_score, out_y, out_x, n_cand, bank_stride, nnz, cluster, subset, ctx->sm_count, &taken),
+                    "correlate");
+  if (taken) return GISAPR_OK;
   GISAPR_CHECK_CUDA(launch_correlate_plain((cudaStream_t)stream, (const float2*)bank, (const float2*)stack,
                                            local_ptr, local_idx, n_particles, n_psi, n, crop, t.outer, t.col,
                                            out_score, out_y, out_x, n_cand, bank_stride, nnz, cluster, subset),
@@ -772,6 +781,12 @@ int gisapr_correlate(gisapr_ctx ctx, void* stream, const float* bank, const floa
   CorrTables t;
   rc = get_corr_tables(ctx, n, crop, &t);
   if (rc) return rc;
+  bool taken;
+  GISAPR_CHECK_CUDA(launch_correlate_rows((cudaStream_t)stream, (const float2*)bank, (const float2*)stack,
+                                          local_ptr, local_idx, n_particles, n_psi, n, crop, t.outer, t.col,
+                                          out_score, out_y, out_x, 1, 0, 0, cluster, nullptr, ctx->sm_count, &taken),
+                    "correlate");
+  if (taken) return GISAPR_OK;
   GISAPR_CHECK_CUDA(launch_correlate_plain((cudaStream_t)stream, (const float2*)bank, (const float2*)stack,
                                            local_ptr, local_idx, n_particles, n_psi, n, crop, t.outer, t.col,
                                            out_score, out_y, out_x, 1, 0, 0, cluster, nullptr),

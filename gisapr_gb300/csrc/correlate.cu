@@ -1,5 +1,7 @@
 // Correlation maximum over the translation window (v606:1418-1449) and the
-// per-particle record statistics (v606:1466-1491), plain FP32, sm_103a.
+// per-particle record statistics (v606:1466-1491), plain FP32, sm_103a. The
+// kernel here takes every size, window and alignment; correlate_rows.cu has a
+// faster form for the sizes and windows that are searched with.
 //
 // For a template T and a particle spectrum P (both stored pre-shifted, packed
 // n x H, H = n/2+1), torch's irfft2 of Q = T * P on the crop window is
