@@ -117,9 +117,14 @@ __host__ __device__ constexpr int twiddle_exponent(int entry) { return (entry / 
 // ``load(g, k)`` gives element k of line g, L.at holds the values between the
 // two steps, ``store(g, k, v)`` takes the result. A load may read any element of
 // the warp's lines (all loads come before the first write). LINES: fewer lines.
-// ``tw`` is the table of twiddle_exponent, in shared memory.
-template <int N, int DIR, int LINES = 0, class Lines, class Load, class Store>
-GISAPR_DEV void line_fft_warp(const Lines& L, const float2* tw, const Load& load, const Store& store) {
+// ``tw`` is the table of twiddle_exponent, in shared memory; ``mul`` multiplies
+// by its entries.
+struct CMul {
+  GISAPR_DEV float2 operator()(float2 a, float2 w) const { return cmul(a, w); }
+};
+template <int N, int DIR, int LINES = 0, class Lines, class Load, class Store, class Mul = CMul>
+GISAPR_DEV void line_fft_warp(const Lines& L, const float2* tw, const Load& load, const Store& store,
+                              const Mul& mul = Mul()) {
   constexpr int L2 = N / 16, G = LINES ? LINES : fft_lines<N>(), T = (G * 16 + 31) / 32;
   const int lane = threadIdx.x & 31;
   {
@@ -136,7 +141,7 @@ GISAPR_DEV void line_fft_warp(const Lines& L, const float2* tw, const Load& load
 #pragma unroll
       for (int k1 = 1; k1 < 16; ++k1) {
         const float2 w = tw[k1 * L2 + n2];
-        L.at(g, L2 * k1 + n2) = cmul(x[k1], DIR < 0 ? w : cconj(w));
+        L.at(g, L2 * k1 + n2) = mul(x[k1], DIR < 0 ? w : cconj(w));
       }
     }
   }
