@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(Rows<C, M, Q>::max_threads, Rows<C, M, Q>::min
               for (int k = 0; k <= h; k += 2) {
                 const float4 u = w[k / 2];
                 A[k] = fmaf(v.x, u.x, A[k]);
-                if (k > 0) B[k] = fmaf(-v.y, u.y, B[k]);  // x = 0: sin 0
+                B[k] = fmaf(-v.y, u.y, B[k]);
                 if (k + 1 <= h) {
                   A[k + 1] = fmaf(v.x, u.z, A[k + 1]);
                   B[k + 1] = fmaf(-v.y, u.w, B[k + 1]);

@@ -741,8 +741,8 @@ __global__ void __launch_bounds__(kRiWarps * 32, 8) rows_inverse(const float2* _
 //
 // Measured before (one CTA of 20 warps per SM on an N x (N + 1) plane of 173 KB
 // at box 128): issue and latency, with every barrier of the one template in
-// flight exposed. The paired rows take 75 KB, so three templates share an SM at
-// box 128 and fill one another's barriers, and the steps between the transforms
+// flight exposed. The paired rows take 75 KB, so two templates of 16 warps share
+// an SM at box 128 and fill one another's barriers, and the steps between the transforms
 // (radial divisor, Hermitian packing, plane removal and mask) run where a
 // transform loads or stores its elements instead of in passes of their own.
 // Column 0 of the plane holds two real columns, DC and Nyquist, and they are
