@@ -4,8 +4,9 @@
 // A thread owns one column of one psi spectrum and Q = 2 or 3 of the residues q
 // of the rows r = M j + q (M = n/16): 16 Q complex values that stay in registers
 // over a group of directions. Per direction it multiplies them by the template's
-// column from shared memory, transforms the 16 rows of each residue, turns the
-// wanted rows by w_n^{q y} and adds its residues up; the L = M/Q lanes that
+// column from shared memory, transforms the 16 rows of each residue, adds the
+// wanted rows of its residues up by powers of w_n^y, which all lanes share, and
+// turns the sum by w_n^{Q l y}; the L = M/Q lanes that
 // share a column then halve the rows among them until each holds the whole sum
 // of C/L rows (an exchange by shuffles that moves every value once). The next
 // template's columns are on their way by asynchronous copies meanwhile. After a
@@ -27,6 +28,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 
 #include "common.cuh"
 
@@ -52,6 +54,7 @@ struct RowsParams {
   int nnz;
   const unsigned char* subset;
   int psi_per_cta;         // blockIdx.y: chunk of psi angles, blockIdx.z: chunk of directions
+  float2 step[16];         // exp(+2 pi i y / n), y = -C/2 ..
 };
 
 template <int C, int M, int Q>
@@ -74,7 +77,7 @@ struct Rows {
   // 12 warps of 168 registers on an SM; 16 of 128 registers spilled and took 1.32 against 1.08 ms
   static constexpr int min_ctas = 12 / (max_threads / 32);
   static size_t smem(int np) {
-    return sizeof(float2) * (2 * (size_t)n * TS + (size_t)M * TWS + (size_t)tile * WS + (size_t)batch * np * C * ZS) +
+    return sizeof(float2) * (2 * (size_t)n * TS + (size_t)L * TWS + (size_t)tile * WS + (size_t)batch * np * C * ZS) +
            sizeof(float) * (size_t)kGroup * np * C * RS;
   }
 };
@@ -102,8 +105,8 @@ __global__ void __launch_bounds__(Rows<C, M, Q>::max_threads, Rows<C, M, Q>::min
   const int K = P.cluster, rank = (int)cluster.block_rank(), b = blockIdx.x / K;
   const int np = P.psi_per_cta, psi0 = blockIdx.y * np, pn = min(np, P.n_psi - psi0);
   float2* s_t = smem;                                        // [2][n][TS]
-  float2* s_two = s_t + 2 * n * TS;                          // [M][TWS]
-  float2* s_twc = s_two + M * R::TWS;                        // [tile][WS]
+  float2* s_two = s_t + 2 * n * TS;                          // [L][TWS]: q = Q l
+  float2* s_twc = s_two + L * R::TWS;                        // [tile][WS]
   float2* s_z = s_twc + tile * WS;                           // [batch][np][C][ZS]
   float* s_raw = reinterpret_cast<float*>(s_z + (size_t)batch * np * C * ZS);  // [kGroup][np][C][RS]
 
@@ -163,7 +166,7 @@ __global__ void __launch_bounds__(Rows<C, M, Q>::max_threads, Rows<C, M, Q>::min
   };
 
   fill(s_group[0], next_cand(0), e0);
-  for (int t = tid; t < M * C; t += blockDim.x) s_two[(t / C) * R::TWS + t % C] = P.tw_outer[t];
+  for (int t = tid; t < L * C; t += blockDim.x) s_two[(t / C) * R::TWS + t % C] = P.tw_outer[(t / C) * Q * C + t % C];
   __syncthreads();
   stage(0, P.bank + s_group[0].src[0], rank * tile);
 
@@ -200,25 +203,31 @@ __global__ void __launch_bounds__(Rows<C, M, Q>::max_threads, Rows<C, M, Q>::min
           stage(buf ^ 1, P.bank + N.src[0], rank * tile);
         const float2* T = s_t + buf * (n * TS) + Q * ql * TS + cl;
         float2 z[CL * L];
+// Z(y) = w^{Q l y} (G_0 + w^y (G_1 + w^y G_2)): w^y is the same in all lanes and comes from the parameters
 #pragma unroll
-        for (int i = 0; i < Q; ++i) {
+        for (int i = Q - 1; i >= 0; --i) {
           float2 x[16];
           const float2* Ti = T + ((Q * ql + i + clo) & 1);
 #pragma unroll
           for (int j = 0; j < 16; ++j) x[j] = cmul(Ti[(M * j + i) * TS], p[i][j]);
           idft16(x);
-          const float2* w = s_two + (Q * ql + i) * R::TWS;
 #pragma unroll
           for (int y = 0; y < C; ++y) {
-            const float2 gq = x[idft16_slot((y - h) & 15)], t = w[y];
-            if (i == 0) {
-              z[y] = cmul(gq, t);
+            const float2 gq = x[idft16_slot((y - h) & 15)], c = P.step[y];
+            if (i == Q - 1) {
+              z[y] = gq;
+            } else if (y == h) {
+              z[y] = cadd(gq, z[y]);
             } else {
-              z[y].x = fmaf(gq.x, t.x, fmaf(-gq.y, t.y, z[y].x));
-              z[y].y = fmaf(gq.x, t.y, fmaf(gq.y, t.x, z[y].y));
+              const float2 v = z[y];
+              z[y].x = fmaf(v.x, c.x, fmaf(-v.y, c.y, gq.x));
+              z[y].y = fmaf(v.x, c.y, fmaf(v.y, c.x, gq.y));
             }
           }
         }
+        const float2* w = s_two + ql * R::TWS;
+#pragma unroll
+        for (int y = 0; y < C; ++y) z[y] = cmul(z[y], w[y]);
 #pragma unroll
         for (int y = C; y < CL * L; ++y) z[y] = make_float2(0.f, 0.f);
         // lane ql ends with rows CL ql ..
@@ -359,6 +368,10 @@ cudaError_t launch(RowsParams P, int sm_count, cudaStream_t st, bool* taken) {
     }
   }
   P.cluster = K;
+  for (int y = 0; y < C; ++y) {
+    const double a = 2.0 * 3.14159265358979323846 * (y - C / 2) / R::n;
+    P.step[y] = make_float2((float)std::cos(a), (float)std::sin(a));
+  }
   ctas *= K;
   // Still few: the maps are spread, first by psi, then by direction.
   if (ctas < slots) chunks = (int)std::min<long long>(P.n_psi, chunks * (slots / ctas));
@@ -394,9 +407,9 @@ cudaError_t launch(RowsParams P, int sm_count, cudaStream_t st, bool* taken) {
 }
 
 // The sizes of the searches. us in this form and in the one of correlate.cu, six
-// directions and three angles: 64 (4,000 particles, window 10) 238 / 533, 96
-// (2,000, 12) 311 / 526, 128 (2,000, 12) 440 / 800, 192 (1,000, 12) 724 / 1397,
-// 256 (500 with eight directions, 14) 1012 / 1526; one particle at 128 8.6 / 24.
+// directions and three angles: 64 (4,000 particles, window 10) 236 / 533, 96
+// (2,000, 12) 307 / 526, 128 (2,000, 12) 442 / 800, 192 (1,000, 12) 716 / 1397,
+// 256 (500 with eight directions, 14) 920 / 1526; one particle at 128 8.7 / 24.
 // Other sizes and windows below 8 stay with the other, which takes any.
 template <int C>
 cudaError_t launch_size(const RowsParams& P, int n, int sm_count, cudaStream_t st, bool* taken) {
