@@ -833,9 +833,9 @@ def run_gb300(args, rank: int, world: int, local_rank: int):
     corr_s = stage_ms["correlate"] / 1e3
     dominant = max(stage_ms, key=stage_ms.get)
     achieved = flops / corr_s / 1e12
-    traffic = profiled_traffic("correlate_plain", args.workload) if not args.particles else None
+    traffic = profiled_traffic("correlate_rows", args.workload) if not args.particles else None
     roofline = {
-        "kernel": "correlate_plain", "bound": "tensor", "achieved": achieved, "peak": bf16_peak,
+        "kernel": "correlate_rows", "bound": "tensor", "achieved": achieved, "peak": bf16_peak,
         "unit": "TFLOP/s", "frac": achieved / bf16_peak, "traffic": traffic,
         "peak_source": f"{peak_kind} bf16 dense (MEASURED_PEAKS.json)" if peak_kind == "measured" else "fallback",
         "algorithmic": f"{flops:.4g} flop per launch = {maps} maps x (6K + 2.5 n^2 log2 n^2), n={cfg.new_box}",
