@@ -19,12 +19,13 @@
 //      centred (z, y) order, blocks of 2 (z) x 4 (y) x 2 (x) voxels of 128
 //      bytes, x padded to N + 2 (the pad column repeats column N).
 // The intermediate arrays (N (N+1) N and 2N (N+1) N complex) stay in L2 at
-// box 128, where the passes take 24, 17 and 30 us (45 us of memory traffic at
-// the copy rate if none of it stayed in L2); at box 256 156, 118 and 234 us
+// box 128, where the passes take 20, 17 and 30 us (45 us of memory traffic at
+// the copy rate if none of it stayed in L2); at box 256 117, 118 and 234 us
 // against 30, 60 and 119. With the lines staged first and every result carried
 // through registers into a second staging they took 25, 26 and 41, and 159, 233
 // and 331: shared-memory round trips between barriers, not traffic. The x pass is
-// bound by the weights (a square root, a sine and a division per voxel).
+// bound by the weights (a square root, a sine and a division), so the two voxels
+// at N/2 - j and N/2 + j share one (24 -> 20 us, 156 -> 117).
 #include "common.cuh"
 #include "pairplane.cuh"
 
@@ -92,14 +93,18 @@ __global__ void __launch_bounds__(PassXY<N>::threads) vfft_x(const float* __rest
   extern __shared__ float2 s_vf[];
   __shared__ float s_row[R][N];
   float2 *s_tw = s_vf, *s_w = s_tw + N, *s_line = s_w + N, *s_out = s_line + (V::threads / 32) * V::stage;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int z = blockIdx.y, y0 = blockIdx.x * R, half = N / 2;
+  constexpr int half = N / 2;
+  const int warp = threadIdx.x >> 5;
+  const int z = blockIdx.y, y0 = blockIdx.x * R;
   const float fz = fftfreq_shifted_f32(z + half, m);
-  for (int idx = lane; idx < D * N; idx += 32) {
-    const int q = warp * D + idx / N, x = idx % N, y = y0 + q;
-    const float fy = fftfreq_shifted_f32(y + half, m), fx = fftfreq_shifted_f32(x + half, m);
+  // the weight at x = N/2 - j and N/2 + j is the same
+  for (int idx = threadIdx.x; idx < R * (half + 1); idx += blockDim.x) {
+    const int q = idx / (half + 1), j = idx % (half + 1), y = y0 + q;
+    const float fy = fftfreq_shifted_f32(y + half, m), fx = fftfreq_shifted_f32(N - j, m);
     const float w = sinc2_f32(__fmul_rn(fz, fz), __fmul_rn(fy, fy), __fmul_rn(fx, fx));
-    s_row[q][x] = __fmul_rn(__ldg(vol + ((size_t)z * N + y) * N + x), w);
+    const float* row = vol + ((size_t)z * N + y) * N;
+    s_row[q][half - j] = __fmul_rn(__ldg(row + half - j), w);
+    if (j > 0 && j < half) s_row[q][half + j] = __fmul_rn(__ldg(row + half + j), w);
   }
   vf_tables<N>(tw_g, s_tw, s_w);
   __syncthreads();
