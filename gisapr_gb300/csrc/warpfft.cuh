@@ -1,17 +1,12 @@
-// Warp-level four-step FFTs on lines staged in shared memory, shared by the
-// projector (project.cu) and the volume transform (volfft.cu).
+// Warp-level four-step FFTs on lines staged in shared memory, as the general
+// projector of box 256 runs them (project.cu).
 #pragma once
 
 #include "common.cuh"
 
-// Row stride (complex elements) of the padded shared-memory plane: holds the
-// N + 1 columns plus one spare slot per 8, chosen by a bank-conflict search.
-// Box 256 has no shared-memory plane; its value there is the stride of
-// rows_inverse's staging lines (256 elements plus one spare slot per 8).
-__host__ __device__ constexpr int plane_ld(int N) {
-  return N == 256 ? 290 : (N == 128 ? 150 : (N == 64 ? 74 : 38));
-}
-__host__ __device__ constexpr int plane_rows(int N) { return N + N / 8; }
+// Stride of a staging line of box 256: 256 elements plus one spare slot per 8,
+// chosen by a bank-conflict search.
+__host__ __device__ constexpr int plane_ld(int N) { return N == 256 ? 290 : 0; }
 
 // Lines of length N with one spare slot per 8 elements, line stride
 // plane_ld(N): element k of line g.
