@@ -9,10 +9,39 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <mutex>
+
 #define GISAPR_DEV __device__ __forceinline__
 
 // Largest 1-D transform length any kernel stages in shared memory.
 constexpr int kMaxFftLen = 512;
+
+// The dynamic shared memory a kernel has been allowed, per device: the runtime
+// keeps the limit of a kernel on the device that is current when it is set. One
+// object per kernel, kept by its launcher.
+struct SmemLimit {
+  static constexpr int kDevices = 64;
+  std::atomic<size_t> bytes[kDevices] = {};
+  std::mutex raising;
+};
+
+// Allows ``kernel`` at least ``smem`` bytes on the current device. The limit is
+// raised once per size, so that a warm launch can be captured in a graph, and is
+// never lowered: another thread may be about to launch with more.
+template <class Kernel>
+cudaError_t allow_smem(Kernel kernel, size_t smem, SmemLimit& limit) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= SmemLimit::kDevices) return cudaErrorInvalidDevice;
+  if (limit.bytes[dev].load() >= smem) return cudaSuccess;
+  std::lock_guard<std::mutex> lock(limit.raising);
+  if (limit.bytes[dev].load() >= smem) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) limit.bytes[dev].store(smem);
+  return e;
+}
 
 // Packed float32 pairs (PTX f32x2): one instruction for both halves, each
 // rounded as its scalar form. The FMA pipes do as many operations a cycle as

@@ -304,13 +304,9 @@ size_t correlate_smem_bytes(int n, int n_psi, int crop, int cluster) {
 
 template <int C>
 static cudaError_t launch_c(const CorrParams& P, size_t smem, cudaStream_t st) {
-  static size_t set_smem = 0;  // attribute set once per size, never inside a stream capture
-  if (set_smem < smem) {
-    cudaError_t e = cudaFuncSetAttribute(correlate_plain<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    set_smem = smem;
-  }
+  static SmemLimit limit;
+  const cudaError_t e = allow_smem(correlate_plain<C>, smem, limit);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(P.n_particles * P.cluster));
   cfg.blockDim = dim3(kThreads);

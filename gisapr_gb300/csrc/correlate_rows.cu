@@ -27,7 +27,6 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 
 #include "common.cuh"
@@ -381,15 +380,9 @@ cudaError_t launch(RowsParams P, int sm_count, cudaStream_t st, bool* taken) {
   const int splits = (int)std::min<long long>(8, std::max<long long>(1, slots / now));
   const size_t smem = R::smem(P.psi_per_cta);
   if (chunks > 65535) return cudaSuccess;
-  static std::atomic<unsigned long long> ready{0};  // devices whose attribute is set
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  static SmemLimit limit;
+  const cudaError_t e = allow_smem(correlate_rows<C, M, Q>, R::smem(kPsi), limit);
   if (e != cudaSuccess) return e;
-  if (dev > 63 || !(ready.load() >> dev & 1)) {
-    e = cudaFuncSetAttribute(correlate_rows<C, M, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::smem(kPsi));
-    if (e != cudaSuccess) return e;
-    if (dev <= 63) ready.fetch_or(1ull << dev);
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(P.n_particles * K), chunks, splits);
   cfg.blockDim = dim3((R::tile * R::L * P.psi_per_cta + 31) / 32 * 32);

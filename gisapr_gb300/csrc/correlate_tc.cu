@@ -828,13 +828,9 @@ __global__ void bank_to_operands(const float2* __restrict__ bank, long long bank
 
 template <int C, int N, bool BF>
 cudaError_t launch_tc_cnb(const TcParams& P, size_t smem, int grid, cudaStream_t st) {
-  static size_t set_smem = 0;
-  if (set_smem < smem) {
-    cudaError_t e =
-        cudaFuncSetAttribute(correlate_tc<C, N, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    set_smem = smem;
-  }
+  static SmemLimit limit;
+  const cudaError_t e = allow_smem(correlate_tc<C, N, BF>, smem, limit);
+  if (e != cudaSuccess) return e;
   correlate_tc<C, N, BF><<<grid, kTcThreads, smem, st>>>(P);
   return cudaGetLastError();
 }
@@ -955,16 +951,10 @@ cudaError_t launch_bank_to_operands(cudaStream_t st, const float2* bank, long lo
   // bank at box 128)
   const int cb = std::min(n / 2 + 1, 16);
   const size_t smem = (size_t)bank_fp16_ld(n) * cb * sizeof(float2);
-  static size_t set_smem[2] = {0, 0};
-  const int k = bf16 ? 1 : 0;
-  if (set_smem[k] < smem) {
-    cudaError_t e = bf16 ? cudaFuncSetAttribute(bank_to_operands<true>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                         : cudaFuncSetAttribute(bank_to_operands<false>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    set_smem[k] = smem;
-  }
+  static SmemLimit limit[2];
+  const cudaError_t e = bf16 ? allow_smem(bank_to_operands<true>, smem, limit[1])
+                             : allow_smem(bank_to_operands<false>, smem, limit[0]);
+  if (e != cudaSuccess) return e;
   if (bf16)
     bank_to_operands<true><<<dim3(n_slot, n_cand), 256, smem, st>>>(bank, bank_stride, n, n_cand, cb, t_scale,
                                                                      (unsigned char*)out, split, status);

@@ -368,10 +368,9 @@ cudaError_t launch_ingest_spectrum(cudaStream_t st, double2* work, int n, int ch
   const size_t amps = (size_t)ch * (cw / 2 + 1) * sizeof(double);
   const bool hold = bin_ptr != nullptr && keep && ch <= 256 && cw <= 256 && bins + ramps + amps <= 200 * 1024;
   const size_t smem = bins + (keep ? ramps : 0) + (hold ? amps : 0);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(ingest_spectrum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  static SmemLimit limit;
+  const cudaError_t e = allow_smem(ingest_spectrum, smem, limit);
+  if (e != cudaSuccess) return e;
   const SpectrumSteps P{bin_ptr, bin_pix, bin_count, n_bins, normalize, plane_sums(ch, cw), keep && normalize ? 1 : 0, hold ? 1 : 0, mask};
   ingest_spectrum<<<n, kSpectrumThreads, smem, st>>>(work, ch, cw, P);
   return cudaGetLastError();

@@ -391,13 +391,9 @@ template <int N>
 cudaError_t launch_plane(const PrepParams& P, int sm_count, cudaStream_t st) {
   const size_t smem = (size_t)(pair_elems(N) + 2 * N) * sizeof(float2) + (prep_threads<N>() / 32 + 1) * sizeof(double) +
                       (size_t)prep_images<N>() * image_elems<N>() * sizeof(float);
-  static size_t set_smem = 0;  // attribute set once, never inside a stream capture
-  if (set_smem < smem) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(prepare_plane<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    set_smem = smem;
-  }
+  static SmemLimit limit;
+  const cudaError_t e = allow_smem(prepare_plane<N>, smem, limit);
+  if (e != cudaSuccess) return e;
   // one CTA per SM at 128 and 192 (the plane and the images fill it), two at
   // 96, five at 64 and as many at 32
   const long long jobs = (long long)P.n * P.n_psi, most = (long long)sm_count * (N >= 128 ? 1 : (N == 96 ? 2 : 5));
@@ -448,13 +444,9 @@ cudaError_t launch_prepare_particles(cudaStream_t st, const float* images, int n
     default: return cudaErrorInvalidValue;
   }
   const size_t smem = prepare_smem_bytes(N);
-  static size_t set_smem = 0;
-  if (set_smem < smem) {
-    cudaError_t e = cudaFuncSetAttribute(prepare_particles, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    set_smem = smem;
-  }
+  static SmemLimit limit;
+  const cudaError_t e = allow_smem(prepare_particles, smem, limit);
+  if (e != cudaSuccess) return e;
   prepare_particles<<<grid, kThreads, smem, st>>>(P);
   return cudaGetLastError();
 }

@@ -1143,14 +1143,6 @@ static size_t tail_smem_bytes(int N, int n_bins) {
   return (size_t)(pair_elems(N) + N) * sizeof(float2) + (size_t)n_bins * sizeof(float);
 }
 
-template <class K>
-static cudaError_t allow_smem(K kernel, size_t smem, size_t& set_smem) {  // once per size, never inside a stream capture
-  if (set_smem >= smem) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) set_smem = smem;
-  return e;
-}
-
 template <int N>
 static cudaError_t launch_planes(ProjParams P, float2* planes, float2* blocked, cudaStream_t st) {
   constexpr int CC = ri_cols<N>();
@@ -1165,9 +1157,9 @@ static cudaError_t launch_planes(ProjParams P, float2* planes, float2* blocked, 
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   P.planes = planes;
-  static size_t set_smem = 0;
+  static SmemLimit limit;
   const size_t smem = tail_smem_bytes(N, P.t.n_bins);
-  e = allow_smem(template_tail<N>, smem, set_smem);
+  e = allow_smem(template_tail<N>, smem, limit);
   if (e != cudaSuccess) return e;
   template_tail<N><<<P.n_build, tail_threads<N>(), smem, st>>>(P);
   return cudaGetLastError();
@@ -1175,9 +1167,9 @@ static cudaError_t launch_planes(ProjParams P, float2* planes, float2* blocked, 
 
 template <int N>
 static cudaError_t launch_general(const ProjParams& P, int grid, cudaStream_t st) {
-  static size_t set_smem = 0;
+  static SmemLimit limit;
   const size_t smem = general_smem_bytes(N, P.t.n_bins);
-  const cudaError_t e = allow_smem(project_templates<N>, smem, set_smem);
+  const cudaError_t e = allow_smem(project_templates<N>, smem, limit);
   if (e != cudaSuccess) return e;
   project_templates<N><<<grid, kThreads, smem, st>>>(P);
   return cudaGetLastError();

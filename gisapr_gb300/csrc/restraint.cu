@@ -144,9 +144,10 @@ size_t edt_smem_bytes(int box) { return (size_t)kTileLines * box * sizeof(int); 
 cudaError_t launch_restraint_edt(cudaStream_t st, const float* density, float threshold, unsigned char* mask,
                                  int* d2, int* scratch, int box) {
   const size_t smem = edt_smem_bytes(box);
-  cudaError_t e = cudaFuncSetAttribute(edt_pass_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemLimit limit_x, limit_yz;
+  cudaError_t e = allow_smem(edt_pass_x, smem, limit_x);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(edt_pass_yz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = allow_smem(edt_pass_yz, smem, limit_yz);
   if (e != cudaSuccess) return e;
   const int tiles = (box + kTileLines - 1) / kTileLines;
   edt_pass_x<<<dim3(tiles, box), kEdtThreads, smem, st>>>(density, threshold, mask, d2, box);

@@ -186,12 +186,11 @@ __global__ void __launch_bounds__(PassZ<N>::threads) vfft_z(const float2* __rest
 }
 
 template <class Kernel, class... Args>
-cudaError_t launch_pass(Kernel kernel, dim3 grid, int threads, int elems, cudaStream_t st, Args... args) {
+cudaError_t launch_pass(Kernel kernel, SmemLimit& limit, dim3 grid, int threads, int elems, cudaStream_t st,
+                        Args... args) {
   const size_t smem = elems * sizeof(float2);
-  if (smem > 40 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = allow_smem(kernel, smem, limit);
+  if (e != cudaSuccess) return e;
   kernel<<<grid, threads, smem, st>>>(args...);
   return cudaGetLastError();
 }
@@ -202,11 +201,12 @@ cudaError_t launch_vfft(cudaStream_t st, const float* vol, float2* a1, float2* a
   using V = PassXY<N>;
   using Z = PassZ<N>;
   static_assert(N % V::lines == 0, "row bands tile the box");
-  cudaError_t e = launch_pass(vfft_x<N>, dim3(N / V::lines, N), V::threads, V::elems(N / 2 + 1), st, vol, a1, tw);
+  static SmemLimit lx, ly, lz;
+  cudaError_t e = launch_pass(vfft_x<N>, lx, dim3(N / V::lines, N), V::threads, V::elems(N / 2 + 1), st, vol, a1, tw);
   if (e != cudaSuccess) return e;
-  e = launch_pass(vfft_y<N>, dim3(N + 1, N / V::lines), V::threads, V::elems(N), st, a1, a2, tw);
+  e = launch_pass(vfft_y<N>, ly, dim3(N + 1, N / V::lines), V::threads, V::elems(N), st, a1, a2, tw);
   if (e != cudaSuccess) return e;
-  return launch_pass(vfft_z<N>, dim3((N + 2) / 2, 2 * N / 4), Z::threads, Z::elems(N), st, a2, blocked, tw);
+  return launch_pass(vfft_z<N>, lz, dim3((N + 2) / 2, 2 * N / 4), Z::threads, Z::elems(N), st, a2, blocked, tw);
 }
 
 }  // namespace
