@@ -1063,7 +1063,10 @@ int gisapr_restraint_poses(gisapr_ctx ctx, void* stream, const float* xyz, const
   if (box < 1 || box > 1024) return fail(GISAPR_ERR_ARGUMENT, "box must be in [1, 1024]");
   if (width < 3) return fail(GISAPR_ERR_ARGUMENT, "width must be >= 3 (insufficient sampling)");
   if (!(apix > 0.0) || !std::isfinite(apix) || !std::isfinite(rp) || !std::isfinite(kn))
-    return fail(GISAPR_ERR_ARGUMENT, "apix, rp and kn must be positive and finite");
+    return fail(GISAPR_ERR_ARGUMENT, "apix must be positive and finite, rp and kn finite");
+  // only bricks that an atom reaches are visited, and below zero every voxel of the bounds is above the threshold
+  if (threshold < 0.0f)
+    return fail(GISAPR_ERR_ARGUMENT, "a threshold below zero needs gisapr_deposit and gisapr_restraint_eval per pose");
   for (int c = 0; c < n_poses; ++c)
     for (int a = 0; a < 3; ++a)
       if (bounds[6 * c + a] < 0 || bounds[6 * c + 3 + a] > box || bounds[6 * c + a] > bounds[6 * c + 3 + a])

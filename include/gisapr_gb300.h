@@ -387,7 +387,8 @@ int gisapr_restraint_eval(gisapr_ctx ctx, void* stream, float* volume, const uns
  * gisapr_deposit does, and reduced against mask and d2 as gisapr_restraint_eval
  * does into out [n_poses][3], which is set here. bounds: per pose {z0, y0, x0,
  * z1, y1, x1} (host memory), half-open, holding every voxel the pose's atoms
- * reach inside the box.
+ * reach inside the box. The threshold is not below zero: there voxels that no
+ * atom reaches count as well, and this call visits none of them.
  */
 int gisapr_restraint_poses(gisapr_ctx ctx, void* stream, const float* xyz, const float* numbers, int n_atoms,
                            int n_poses, const int* bounds, const unsigned char* mask, const int* d2, int box, int width,
