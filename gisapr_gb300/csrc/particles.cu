@@ -217,14 +217,6 @@ __device__ __forceinline__ float2 div_nm1(float2 a) {
   return fma2(fma2(q, dup2(-d), a), dup2(r), q);
 }
 
-// s + c += x * x in two floats (48 bits): GB300's FP64 rate is 1/64 of its
-// FP32 rate, and the L2 norm's FP64 sums took as long as the transforms.
-__device__ __forceinline__ void add_square(float x, float& s, float& c) {
-  const float t = __fmaf_rn(x, x, s);
-  c = __fadd_rn(c, __fmaf_rn(x, x, -__fsub_rn(t, s)));
-  s = t;
-}
-
 __device__ __forceinline__ float small_to_float(int i) {  // 0 <= i < 2^23, FP32 pipe
   return __int_as_float(0x4B000000 | i) - 8388608.0f;
 }
@@ -342,7 +334,7 @@ __global__ void __launch_bounds__(prep_threads<N>(), N <= 64 ? 4 : (N == 96 ? 2 
     // nb / 2 in s_last) and squared for the norm, then scaled and written
     const float* ctf = P.ctf + (size_t)p * nb * H;
     const int hb = nb / 2;
-    float hi = 0.f, lo = 0.f;
+    float2 hi = make_float2(0.f, 0.f), lo = hi;  // the L2 norm; in FP64 it took as long as the transforms
     for (int r = warp; r < nb; r += NW) {
       const int i = r < hb ? r : r + N - nb;
 #pragma unroll 2
@@ -350,8 +342,7 @@ __global__ void __launch_bounds__(prep_threads<N>(), N <= 64 ? 4 : (N == 96 ? 2 
         float2& z = Z.half(i, c);
         const float2 f = cscale(cconj(z), __ldg(ctf + r * H + c));
         z = f;
-        add_square(f.x, hi, lo);
-        add_square(f.y, hi, lo);
+        add_squares(f, hi, lo);
       }
     }
     for (int r = tid; r < nb; r += NT) {
@@ -361,10 +352,9 @@ __global__ void __launch_bounds__(prep_threads<N>(), N <= 64 ? 4 : (N == 96 ? 2 
       const float2 z = nb == N ? cconj(s_last[i]) : Z.half(i == 0 ? 0 : N - i, hb);
       const float2 f = cscale(z, __ldg(ctf + r * H + hb));
       s_last[r] = f;
-      add_square(f.x, hi, lo);
-      add_square(f.y, hi, lo);
+      add_squares(f, hi, lo);
     }
-    const double ss = warp_sum_d((double)hi + (double)lo);
+    const double ss = warp_sum_d(squares_total(hi, lo));
     if (lane == 0) red[warp] = ss;
     __syncthreads();
     if (tid == 0) {  // one thread: FP64 division and square root
