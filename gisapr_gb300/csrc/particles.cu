@@ -15,6 +15,7 @@
 // plane does not fit an SM, through a global scratch plane.
 #include "common.cuh"
 #include "pairplane.cuh"
+#include "rotate.cuh"
 
 namespace {
 
@@ -72,24 +73,6 @@ struct PrepParams {
   const float2* tw3;       // twiddles of lengths 3 * 2^k
   int n, n_psi, N, nb;
 };
-
-__device__ __forceinline__ float sample_bilinear_zero(const float* __restrict__ img, int N,
-                                                      float iy, float ix) {
-  const float fy = floorf(iy), fx = floorf(ix);
-  const int y0 = (int)fy, x0 = (int)fx;
-  const float w = __fsub_rn(ix, fx), e = __fsub_rn(1.0f, w);
-  const float nn = __fsub_rn(iy, fy), s = __fsub_rn(1.0f, nn);
-  const float wnw = __fmul_rn(s, e), wne = __fmul_rn(s, w);
-  const float wsw = __fmul_rn(nn, e), wse = __fmul_rn(nn, w);
-  auto at = [&](int yy, int xx) -> float {
-    return (yy >= 0 && yy < N && xx >= 0 && xx < N) ? __ldg(img + (size_t)yy * N + xx) : 0.0f;
-  };
-  float acc = __fmul_rn(at(y0, x0), wnw);
-  acc = __fadd_rn(acc, __fmul_rn(at(y0, x0 + 1), wne));
-  acc = __fadd_rn(acc, __fmul_rn(at(y0 + 1, x0), wsw));
-  acc = __fadd_rn(acc, __fmul_rn(at(y0 + 1, x0 + 1), wse));
-  return acc;
-}
 
 __global__ void __launch_bounds__(kThreads) prepare_particles(PrepParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -202,24 +185,8 @@ template <int N>
 __host__ __device__ constexpr int prep_threads() { return N <= 64 ? 128 : (N == 96 ? 384 : (N == 128 ? 512 : 768)); }
 template <int N>
 __host__ __device__ constexpr int prep_images() { return N == 128 ? 2 : (N < 128 ? 1 : 0); }
-constexpr int kBorder = 2;
-template <int N>
-__host__ __device__ constexpr int image_ld() { return N + 9; }
 template <int N>
 __host__ __device__ constexpr int image_elems() { return (N + 2 * kBorder) * image_ld<N>(); }
-
-// a / (N - 1), correctly rounded: one Newton correction of a * RN(1 / (N - 1))
-// (Markstein's theorem; the remainder is exact in the fused multiply-add).
-template <int N>
-__device__ __forceinline__ float2 div_nm1(float2 a) {
-  constexpr float d = (float)(N - 1), r = 1.0f / (float)(N - 1);
-  const float2 q = mul2(a, dup2(r));
-  return fma2(fma2(q, dup2(-d), a), dup2(r), q);
-}
-
-__device__ __forceinline__ float small_to_float(int i) {  // 0 <= i < 2^23, FP32 pipe
-  return __int_as_float(0x4B000000 | i) - 8388608.0f;
-}
 
 template <int N>
 __global__ void __launch_bounds__(prep_threads<N>(), N <= 64 ? 4 : (N == 96 ? 2 : 1)) prepare_plane(PrepParams P) {
@@ -255,7 +222,6 @@ __global__ void __launch_bounds__(prep_threads<N>(), N <= 64 ? 4 : (N == 96 ? 2 
   __syncthreads();  // the zeroed border before the copies
   if (NI > 0 && p0 <= p1) load_image(p0);
   int ready = p0 - 1;  // the last image that has been waited for
-  const float half = __fdiv_rn((float)(N - 1), 2.0f);
   // lanes take 8 columns x 4 row pairs of the rotated image: a compact footprint
   const int lj = tid & 7, lq = (tid >> 3) & 3;
   constexpr int JT = N / 8, QT = N / 8;  // tiles of 8 columns, of 4 row pairs
@@ -273,45 +239,12 @@ __global__ void __launch_bounds__(prep_threads<N>(), N <= 64 ? 4 : (N == 96 ? 2 
       __syncthreads();
     }
     const float4 ps = P.psi_tab[P.psi_index[(size_t)p * P.n_psi + si]];
-    const float cth = ps.x, sth = ps.y;
     const float* img = NI > 0 ? s_img + (NI > 1 ? ((p - p0) % NI) * IEL : 0) : P.images + (size_t)p * N * N;
 #pragma unroll 2
     for (int tile = warp; tile < JT * QT; tile += NW) {
       // the two rows of a pair, as the halves of packed operations
       const int q = (tile / JT) * 4 + lq, j = (tile % JT) * 8 + lj;
-      const float xx = small_to_float(j), y0f = small_to_float(2 * q);
-      const float2 yy = make_float2(y0f, y0f + 1.0f);
-      // source = [row, col] @ M^T + offset; M = [[c, -s], [s, c]]
-      const float2 sy = add2(fma2(dup2(-sth), dup2(xx), mul2(dup2(cth), yy)), dup2(ps.z));
-      const float2 sx = add2(fma2(dup2(cth), dup2(xx), mul2(dup2(sth), yy)), dup2(ps.w));
-      const float2 yn = add2(div_nm1<N>(mul2(dup2(2.0f), sy)), dup2(-1.0f));
-      const float2 xn = add2(div_nm1<N>(mul2(dup2(2.0f), sx)), dup2(-1.0f));
-      const float2 iy = mul2(add2(yn, dup2(1.0f)), dup2(half)), ix = mul2(add2(xn, dup2(1.0f)), dup2(half));
-      float2 v;
-      if constexpr (NI > 0) {
-        // floor by adding 1.5 * 2^23 rounded down: the sum's low bits are the
-        // integer, clamped as they are (the bits of positive floats are ordered)
-        constexpr float kMagic = 12582912.0f;
-        constexpr int kZero = 0x4B400000;  // the bits of kMagic
-        const float2 ry = add2_down(iy, dup2(kMagic)), rx = add2_down(ix, dup2(kMagic));
-        const float2 fy = add2(ry, dup2(-kMagic)), fx = add2(rx, dup2(-kMagic));
-        const float2 w = sub2(ix, fx), ea = sub2(dup2(1.0f), w);
-        const float2 nn = sub2(iy, fy), s = sub2(dup2(1.0f), nn);
-        auto at = [&](float yb, float xb) {
-          const int y0 = min(max(__float_as_int(yb), kZero - kBorder), kZero + N);
-          const int x0 = min(max(__float_as_int(xb), kZero - kBorder), kZero + N);
-          return img + ((y0 - kZero + kBorder) * ILD + (x0 - kZero + kBorder));
-        };
-        const float* a = at(ry.x, rx.x);
-        const float* b = at(ry.y, rx.y);
-        v = mul2(make_float2(a[0], b[0]), mul2(s, ea));
-        v = add2(v, mul2(make_float2(a[1], b[1]), mul2(s, w)));
-        v = add2(v, mul2(make_float2(a[ILD], b[ILD]), mul2(nn, ea)));
-        v = add2(v, mul2(make_float2(a[ILD + 1], b[ILD + 1]), mul2(nn, w)));
-      } else {
-        v.x = sample_bilinear_zero(img, N, iy.x, ix.x);
-        v.y = sample_bilinear_zero(img, N, iy.y, ix.y);
-      }
+      float2 v = rotated_pair<N, (NI > 0)>(img, ps, q, j);
       if (P.mask != nullptr) {
         const float* mk = P.mask + 2 * q * N + j;
         v = mul2(v, make_float2(__ldg(mk), __ldg(mk + N)));
