@@ -134,7 +134,6 @@ struct IngestPlan {
   int ch = 0, cw = 0, n = 0;
   cufftHandle forward = 0, inverse = 0;
   cudaEvent_t done = nullptr;    // the last call's transforms have run
-  cudaStream_t stream = nullptr; // and where
   unsigned long long used = 0;   // for the choice of the one to give up
 };
 constexpr int kIngestPlans = 4;
@@ -292,9 +291,11 @@ int get_bins(gisapr_ctx ctx, int N, BinTable* out) {
 
 // The plans of ch x cw x n, kept with the context: making them took 0.4 ms of a
 // call and destroying them a wait for the stream. A fifth shape replaces the one
-// used longest ago. A plan's work area is one per plan, so a call on another
-// stream waits for the last one.
-int get_ingest_plan(gisapr_ctx ctx, int ch, int cw, int n, cudaStream_t st, IngestPlan** out) {
+// used longest ago. A plan's work area is one per plan, so a call waits for the
+// last one, whatever its stream: the handle of a destroyed stream may come back
+// for a new one while the old one's work still runs. A capture cannot wait for
+// work outside it; whoever replays it orders it.
+int get_ingest_plan(gisapr_ctx ctx, int ch, int cw, int n, cudaStream_t st, bool capturing, IngestPlan** out) {
   IngestPlan* p = nullptr;
   for (auto& e : ctx->ingest)
     if (e.ch == ch && e.cw == cw && e.n == n) p = &e;
@@ -309,7 +310,7 @@ int get_ingest_plan(gisapr_ctx ctx, int ch, int cw, int n, cudaStream_t st, Inge
       ctx->ingest.erase(old);
     }
     IngestPlan e;
-    e.ch = ch; e.cw = cw; e.n = n; e.stream = st;
+    e.ch = ch; e.cw = cw; e.n = n;
     int dims[2] = {ch, cw}, real[2] = {ch, 2 * (cw / 2 + 1)}, half[2] = {ch, cw / 2 + 1};
     const int dr = real[0] * real[1], dh = half[0] * half[1];
     cufftResult r = cufftPlanMany(&e.forward, 2, dims, real, 1, dr, half, 1, dh, CUFFT_D2Z, n);
@@ -329,8 +330,7 @@ int get_ingest_plan(gisapr_ctx ctx, int ch, int cw, int n, cudaStream_t st, Inge
     ctx->ingest.push_back(e);
     p = &ctx->ingest.back();
   }
-  if (p->stream != st) GISAPR_CHECK_CUDA(cudaStreamWaitEvent(st, p->done, 0), "cudaStreamWaitEvent(ingest)");
-  p->stream = st;
+  if (!capturing) GISAPR_CHECK_CUDA(cudaStreamWaitEvent(st, p->done, 0), "cudaStreamWaitEvent(ingest)");
   p->used = ++ctx->ingest_calls;
   cufftSetStream(p->forward, st);
   cufftSetStream(p->inverse, st);
@@ -995,8 +995,12 @@ int gisapr_ingest_stack(gisapr_ctx ctx, void* stream, const float* images, int n
   // the caller's ch * cw complex values always hold
   const int ld = (flags & 5) ? 2 * (cw / 2 + 1) : cw;
   IngestPlan* plan = nullptr;
+  bool capturing = false;
   if (flags & 5) {
-    rc = get_ingest_plan(ctx, ch, cw, n, st, &plan);
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    GISAPR_CHECK_CUDA(cudaStreamIsCapturing(st, &status), "cudaStreamIsCapturing");
+    capturing = status != cudaStreamCaptureStatusNone;
+    rc = get_ingest_plan(ctx, ch, cw, n, st, capturing, &plan);
     if (rc) return rc;
   }
   GISAPR_CHECK_CUDA(launch_ingest_load(st, images, n, h, w, shifts, ch, cw, work, ld, ctx->sm_count), "ingest_load");
@@ -1009,7 +1013,7 @@ int gisapr_ingest_stack(gisapr_ctx ctx, void* stream, const float* images, int n
                       "ingest_spectrum");
     r = cufftExecZ2D(plan->inverse, (cufftDoubleComplex*)work, (cufftDoubleReal*)work);
     if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecZ2D failed");
-    GISAPR_CHECK_CUDA(cudaEventRecord(plan->done, st), "cudaEventRecord(ingest)");
+    if (!capturing) GISAPR_CHECK_CUDA(cudaEventRecord(plan->done, st), "cudaEventRecord(ingest)");
   } else if (flags & 2) {
     GISAPR_CHECK_CUDA(launch_ingest_normalize(st, work, n, ch, cw, ld), "ingest_normalize");
   }

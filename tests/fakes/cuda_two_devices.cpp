@@ -15,6 +15,7 @@ thread_local int current = 0;
 std::mutex guard;
 std::map<std::pair<int, const void*>, size_t> limits;
 int launched = 0, refused = 0, lowered = 0;
+int recorded = 0, waited = 0;  // events
 
 cudaError_t check(const void* kernel, size_t smem) {
   std::lock_guard<std::mutex> lock(guard);
@@ -34,6 +35,8 @@ extern "C" {
 int fake_launched() { return launched; }
 int fake_refused() { return refused; }
 int fake_lowered() { return lowered; }
+int fake_recorded() { return recorded; }
+int fake_waited() { return waited; }
 
 cudaError_t cudaGetDeviceCount(int* n) { *n = 2; return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { current = d; return cudaSuccess; }
@@ -42,10 +45,10 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 152; retu
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) { *s = cudaStreamCaptureStatusNone; return cudaSuccess; }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { ++waited; return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = nullptr; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { ++recorded; return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) { *p = calloc(1, n); return *p ? cudaSuccess : cudaErrorMemoryAllocation; }

@@ -1,26 +1,9 @@
 """The dynamic shared memory a kernel may take belongs to a device, and a process may hold contexts on several: every
 launcher raises it on the device it launches on, and never lowers it (another thread's larger launch may be on its
 way). Run on a fake CUDA runtime of two devices (fakes/cuda_two_devices.cpp), no kernel runs."""
-import os
-import subprocess
-import sys
-from pathlib import Path
-
-import pytest
-
-ROOT = Path(__file__).resolve().parent.parent
+from .fakes.runtime import run_on_fake
 
 CHILD = r"""
-import ctypes as C, sys
-fake, lib = C.CDLL(sys.argv[1]), C.CDLL(sys.argv[2])
-from gisapr_gb300 import _native as nat
-for name, args in nat.SIGNATURES.items():
-    getattr(lib, name).argtypes = args
-lib.gisapr_last_error.restype = C.c_char_p
-memory = C.create_string_buffer(1 << 20)
-p = C.c_void_p((C.addressof(memory) + 255) & ~255)
-def ok(rc, what):
-    assert rc == 0, (what, lib.gisapr_last_error())
 contexts = []
 for dev in (0, 1):
     c = C.c_void_p()
@@ -57,14 +40,4 @@ print("calls", count)
 
 
 def test_every_launcher_raises_the_limit_on_its_device(native_lib, tmp_path):
-    from gisapr_gb300 import _native
-    from gisapr_gb300.build_native import cuda_home
-    fake = tmp_path / "libfake.so"
-    r = subprocess.run(["g++", "-shared", "-fPIC", "-O1", "-std=c++17", "-I", str(cuda_home() / "include"), "-o", str(fake),
-                        str(ROOT / "tests" / "fakes" / "cuda_two_devices.cpp")], capture_output=True, text=True)
-    assert r.returncode == 0, r.stderr
-    env = dict(os.environ, LD_PRELOAD=str(fake), PYTHONPATH=str(ROOT))
-    r = subprocess.run([sys.executable, "-c", CHILD, str(fake), str(_native.LIB_PATH)], env=env, cwd=str(ROOT),
-                       capture_output=True, text=True, timeout=600)
-    assert r.returncode == 0, r.stdout + r.stderr
-    assert r.stdout.startswith("calls ")
+    assert run_on_fake(CHILD, tmp_path).startswith("calls ")
