@@ -133,10 +133,13 @@ struct CorrTables {
 struct IngestPlan {
   int ch = 0, cw = 0, n = 0;
   cufftHandle forward = 0, inverse = 0;
-  cudaEvent_t done = nullptr;    // the last call's transforms have run
+  size_t work = 0;               // bytes of work area that either takes
+  void* area = nullptr;          // the one they were last given
+  bool captured = false;         // a graph holds them
   unsigned long long used = 0;   // for the choice of the one to give up
 };
 constexpr int kIngestPlans = 4;
+constexpr size_t kIngestKeep = (size_t)1 << 30;  // a larger work area is given back after the call
 
 }  // namespace
 
@@ -150,10 +153,13 @@ struct gisapr_context {
   float2* tw3 = nullptr;  // exp(-2 pi i t / kMaxFftLen3), t < kMaxFftLen3 (lengths 3 * 2^k)
   std::map<int, std::pair<cufftHandle, float*>> fft;  // box -> (R2C plan, padded input)
   std::map<int, BinTable> bins;                        // N -> radial bins
-  std::vector<IngestPlan> ingest;                      // at most kIngestPlans
+  std::vector<IngestPlan> ingest;                      // at most kIngestPlans, and those that graphs hold
   unsigned long long ingest_calls = 0;
+  cudaEvent_t ingest_done = nullptr;                   // the last call's transforms have run
+  bool ingest_captured = false;                        // a graph holds the work area
   std::map<std::pair<int, int>, CorrTables> corr;      // (n, crop) -> twiddles
   DeviceBuffer atoms, bin_counts, bin_lists, proj_scratch, prep_scratch, proj_slices, proj_blocked, vfft_scratch;
+  DeviceBuffer ingest_work;        // of all the kept transforms (they never run at once)
   DeviceBuffer proj_status;        // int: set to 1 by a projector plane wait that ran out
   unsigned proj_wait = 1u << 24;   // bound of that wait (attempts)
   int blocked_box = 0;  // box of the blocked spectrum gisapr_volume_spectrum_blocked last wrote (0: none)
@@ -291,50 +297,99 @@ int get_bins(gisapr_ctx ctx, int N, BinTable* out) {
 
 // The plans of ch x cw x n, kept with the context: making them took 0.4 ms of a
 // call and destroying them a wait for the stream. A fifth shape replaces the one
-// used longest ago. A plan's work area is one per plan, so a call waits for the
-// last one, whatever its stream: the handle of a destroyed stream may come back
-// for a new one while the old one's work still runs. A capture cannot wait for
-// work outside it; whoever replays it orders it.
+// used longest ago. All plans share one work area (each of its own held as much as
+// a batch's spectra, twice for each of the shapes), so a call waits for the last
+// one, whatever its stream: the handle of a destroyed stream may come back for a
+// new one while the old one's work still runs. A capture cannot wait for work
+// outside it; whoever replays it orders it, and what it holds stays with the context.
 int get_ingest_plan(gisapr_ctx ctx, int ch, int cw, int n, cudaStream_t st, bool capturing, IngestPlan** out) {
+  if (ctx->ingest_done == nullptr)
+    GISAPR_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->ingest_done, cudaEventDisableTiming), "cudaEventCreate(ingest)");
   IngestPlan* p = nullptr;
   for (auto& e : ctx->ingest)
     if (e.ch == ch && e.cw == cw && e.n == n) p = &e;
   if (p == nullptr) {
-    if ((int)ctx->ingest.size() == kIngestPlans) {
-      auto old = std::min_element(ctx->ingest.begin(), ctx->ingest.end(),
-                                  [](const IngestPlan& a, const IngestPlan& b) { return a.used < b.used; });
-      cudaEventSynchronize(old->done);
+    auto old = ctx->ingest.end();
+    int kept = 0;
+    for (auto e = ctx->ingest.begin(); e != ctx->ingest.end(); ++e) {
+      if (e->captured) continue;
+      ++kept;
+      if (old == ctx->ingest.end() || e->used < old->used) old = e;
+    }
+    if (kept >= kIngestPlans) {
+      cudaEventSynchronize(ctx->ingest_done);
       cufftDestroy(old->forward);
       cufftDestroy(old->inverse);
-      cudaEventDestroy(old->done);
       ctx->ingest.erase(old);
     }
     IngestPlan e;
     e.ch = ch; e.cw = cw; e.n = n;
     int dims[2] = {ch, cw}, real[2] = {ch, 2 * (cw / 2 + 1)}, half[2] = {ch, cw / 2 + 1};
     const int dr = real[0] * real[1], dh = half[0] * half[1];
-    cufftResult r = cufftPlanMany(&e.forward, 2, dims, real, 1, dr, half, 1, dh, CUFFT_D2Z, n);
+    size_t work[2] = {0, 0};
+    auto make = [&](cufftHandle* h, cufftType type, size_t* bytes) {
+      cufftResult r = cufftCreate(h);
+      if (r != CUFFT_SUCCESS) return r;
+      r = cufftSetAutoAllocation(*h, 0);
+      if (r == CUFFT_SUCCESS)
+        r = type == CUFFT_D2Z ? cufftMakePlanMany(*h, 2, dims, real, 1, dr, half, 1, dh, type, n, bytes)
+                              : cufftMakePlanMany(*h, 2, dims, half, 1, dh, real, 1, dr, type, n, bytes);
+      if (r != CUFFT_SUCCESS) cufftDestroy(*h);
+      return r;
+    };
+    cufftResult r = make(&e.forward, CUFFT_D2Z, &work[0]);
     if (r != CUFFT_SUCCESS)
-      return fail(GISAPR_ERR_CUFFT, "cufftPlanMany(D2Z) failed with code " + std::to_string((int)r));
-    r = cufftPlanMany(&e.inverse, 2, dims, half, 1, dh, real, 1, dr, CUFFT_Z2D, n);
+      return fail(GISAPR_ERR_CUFFT, "cufftMakePlanMany(D2Z) failed with code " + std::to_string((int)r));
+    r = make(&e.inverse, CUFFT_Z2D, &work[1]);
     if (r != CUFFT_SUCCESS) {
       cufftDestroy(e.forward);
-      return fail(GISAPR_ERR_CUFFT, "cufftPlanMany(Z2D) failed with code " + std::to_string((int)r));
+      return fail(GISAPR_ERR_CUFFT, "cufftMakePlanMany(Z2D) failed with code " + std::to_string((int)r));
     }
-    const cudaError_t err = cudaEventCreateWithFlags(&e.done, cudaEventDisableTiming);
-    if (err != cudaSuccess) {
-      cufftDestroy(e.forward);
-      cufftDestroy(e.inverse);
-      return cuda_fail(err, "cudaEventCreate(ingest)");
-    }
+    e.work = std::max<size_t>(16, std::max(work[0], work[1]));
     ctx->ingest.push_back(e);
     p = &ctx->ingest.back();
   }
-  if (!capturing) GISAPR_CHECK_CUDA(cudaStreamWaitEvent(st, p->done, 0), "cudaStreamWaitEvent(ingest)");
+  if (ctx->ingest_work.bytes < p->work) {
+    if (capturing)
+      return fail(GISAPR_ERR_UNSUPPORTED, "a captured preparation needs its work area (1 GB at most) from an earlier call");
+    DeviceBuffer& b = ctx->ingest_work;
+    if (b.ptr != nullptr) {
+      cudaEventSynchronize(ctx->ingest_done);
+      if (ctx->ingest_captured) ctx->retired.push_back(b.ptr);
+      else cudaFree(b.ptr);
+    }
+    b.ptr = nullptr;
+    b.bytes = 0;
+    GISAPR_CHECK_CUDA(cudaMalloc(&b.ptr, p->work), "cudaMalloc(ingest transforms)");
+    b.bytes = p->work;
+  }
+  if (!capturing) GISAPR_CHECK_CUDA(cudaStreamWaitEvent(st, ctx->ingest_done, 0), "cudaStreamWaitEvent(ingest)");
+  if (capturing) p->captured = ctx->ingest_captured = true;
   p->used = ++ctx->ingest_calls;
-  cufftSetStream(p->forward, st);
-  cufftSetStream(p->inverse, st);
+  for (cufftHandle h : {p->forward, p->inverse}) {
+    cufftSetStream(h, st);
+    if (p->area != ctx->ingest_work.ptr) {
+      const cufftResult r = cufftSetWorkArea(h, ctx->ingest_work.ptr);
+      if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftSetWorkArea failed with code " + std::to_string((int)r));
+    }
+  }
+  p->area = ctx->ingest_work.ptr;
   *out = p;
+  return GISAPR_OK;
+}
+
+// After a call's transforms: the mark that the next call waits for, and a large
+// work area is given back.
+int end_ingest_plan(gisapr_ctx ctx, cudaStream_t st, bool capturing) {
+  if (capturing) return GISAPR_OK;
+  GISAPR_CHECK_CUDA(cudaEventRecord(ctx->ingest_done, st), "cudaEventRecord(ingest)");
+  if (ctx->ingest_work.bytes > kIngestKeep && !ctx->ingest_captured) {
+    cudaEventSynchronize(ctx->ingest_done);
+    cudaFree(ctx->ingest_work.ptr);
+    ctx->ingest_work.ptr = nullptr;
+    ctx->ingest_work.bytes = 0;
+    for (auto& e : ctx->ingest) e.area = nullptr;
+  }
   return GISAPR_OK;
 }
 
@@ -450,7 +505,9 @@ int gisapr_context_destroy(gisapr_ctx ctx) {
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
   for (auto& kv : ctx->fft) { cufftDestroy(kv.second.first); cudaFree(kv.second.second); }
-  for (auto& p : ctx->ingest) { cufftDestroy(p.forward); cufftDestroy(p.inverse); cudaEventDestroy(p.done); }
+  for (auto& p : ctx->ingest) { cufftDestroy(p.forward); cufftDestroy(p.inverse); }
+  if (ctx->ingest_done != nullptr) cudaEventDestroy(ctx->ingest_done);
+  cudaFree(ctx->ingest_work.ptr);
   for (auto& kv : ctx->bins) {
     cudaFree(kv.second.list); cudaFree(kv.second.off); cudaFree(kv.second.ptr); cudaFree(kv.second.count);
     cudaFree(kv.second.tw);
@@ -1005,15 +1062,20 @@ int gisapr_ingest_stack(gisapr_ctx ctx, void* stream, const float* images, int n
   }
   GISAPR_CHECK_CUDA(launch_ingest_load(st, images, n, h, w, shifts, ch, cw, work, ld, ctx->sm_count), "ingest_load");
   if (flags & 5) {
-    cufftResult r = cufftExecD2Z(plan->forward, (cufftDoubleReal*)work, (cufftDoubleComplex*)work);
-    if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecD2Z failed");
-    GISAPR_CHECK_CUDA(launch_ingest_spectrum(st, (double2*)work, n, ch, cw, (flags & 1) ? bin_ptr : nullptr, bin_pix,
-                                             bin_count, n_bins, (flags & 2) ? 1 : 0,
-                                             (flags & 4) ? highpass_mask : nullptr),
-                      "ingest_spectrum");
-    r = cufftExecZ2D(plan->inverse, (cufftDoubleComplex*)work, (cufftDoubleReal*)work);
-    if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecZ2D failed");
-    if (!capturing) GISAPR_CHECK_CUDA(cudaEventRecord(plan->done, st), "cudaEventRecord(ingest)");
+    auto transforms = [&]() -> int {
+      cufftResult r = cufftExecD2Z(plan->forward, (cufftDoubleReal*)work, (cufftDoubleComplex*)work);
+      if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecD2Z failed");
+      GISAPR_CHECK_CUDA(launch_ingest_spectrum(st, (double2*)work, n, ch, cw, (flags & 1) ? bin_ptr : nullptr, bin_pix,
+                                               bin_count, n_bins, (flags & 2) ? 1 : 0,
+                                               (flags & 4) ? highpass_mask : nullptr),
+                        "ingest_spectrum");
+      r = cufftExecZ2D(plan->inverse, (cufftDoubleComplex*)work, (cufftDoubleReal*)work);
+      if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecZ2D failed");
+      return GISAPR_OK;
+    };
+    rc = transforms();
+    const int ended = end_ingest_plan(ctx, st, capturing);
+    if (rc || ended) return rc ? rc : ended;
   } else if (flags & 2) {
     GISAPR_CHECK_CUDA(launch_ingest_normalize(st, work, n, ch, cw, ld), "ingest_normalize");
   }

@@ -347,9 +347,11 @@ int gisapr_score_sum_batch(void* stream, const int* local_ptr, const float* peak
  * normalisation (normalize), 4 = high-pass by highpass_mask (ch*cw doubles,
  * unshifted order, radial). Bins and mask depend on the centred radius alone:
  * the steps run in the half spectrum of real images. The context keeps the
- * transform plans of the last four (ch, cw, n).
+ * transform plans of the last four (ch, cw, n) and one work area for all of
+ * them, as large as the largest needs; one above 1 GB is given back after the
+ * call, which then waits for it.
  * work: n*ch*cw*2 doubles; out: n float32 ch x cw images.
- * Every pointer but shifts is device memory.
+ * Every pointer is device memory.
  */
 int gisapr_ingest_stack(gisapr_ctx ctx, void* stream, const float* images, int n, int h, int w, const int* shifts,
                         int ch, int cw, int flags, const int* bin_ptr, const int* bin_pix, const double* bin_count,

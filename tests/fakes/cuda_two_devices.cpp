@@ -16,6 +16,18 @@ std::mutex guard;
 std::map<std::pair<int, const void*>, size_t> limits;
 int launched = 0, refused = 0, lowered = 0;
 int recorded = 0, waited = 0;  // events
+size_t held = 0, plan_held = 0, plan_bytes = 1024;  // device memory of the callers and of plans; what a plan takes
+std::map<void*, size_t> sizes;
+std::map<int, size_t> plans;  // handle -> work area of its own
+std::map<int, bool> automatic;
+int last_plan = 0;
+
+cufftResult plan_made(int h) {
+  if (automatic.count(h) && !automatic[h]) return CUFFT_SUCCESS;
+  plans[h] = plan_bytes;
+  plan_held += plan_bytes;
+  return CUFFT_SUCCESS;
+}
 
 cudaError_t check(const void* kernel, size_t smem) {
   std::lock_guard<std::mutex> lock(guard);
@@ -37,6 +49,8 @@ int fake_refused() { return refused; }
 int fake_lowered() { return lowered; }
 int fake_recorded() { return recorded; }
 int fake_waited() { return waited; }
+long long fake_held() { return (long long)(held + plan_held); }
+void fake_plan_bytes(long long n) { plan_bytes = (size_t)n; }
 
 cudaError_t cudaGetDeviceCount(int* n) { *n = 2; return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { current = d; return cudaSuccess; }
@@ -51,8 +65,19 @@ cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { ++recorded; return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
-cudaError_t cudaMalloc(void** p, size_t n) { *p = calloc(1, n); return *p ? cudaSuccess : cudaErrorMemoryAllocation; }
-cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) {  // no more than 1 MB of it is there
+  *p = calloc(1, n < (1 << 20) ? n : 1 << 20);
+  if (*p == nullptr) return cudaErrorMemoryAllocation;
+  sizes[*p] = n;
+  held += n;
+  return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+  held -= sizes[p];
+  sizes.erase(p);
+  free(p);
+  return cudaSuccess;
+}
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemset(void*, int, size_t) { return cudaSuccess; }
@@ -77,18 +102,18 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* kernel,
   return check(kernel, c->dynamicSmemBytes);
 }
 
-cufftResult cufftCreate(cufftHandle* h) { *h = 1; return CUFFT_SUCCESS; }
-cufftResult cufftDestroy(cufftHandle) { return CUFFT_SUCCESS; }
+cufftResult cufftCreate(cufftHandle* h) { *h = ++last_plan; return CUFFT_SUCCESS; }
+cufftResult cufftDestroy(cufftHandle h) { plan_held -= plans[h]; plans.erase(h); return CUFFT_SUCCESS; }
 cufftResult cufftSetStream(cufftHandle, cudaStream_t) { return CUFFT_SUCCESS; }
-cufftResult cufftSetAutoAllocation(cufftHandle, int) { return CUFFT_SUCCESS; }
+cufftResult cufftSetAutoAllocation(cufftHandle h, int on) { automatic[h] = on != 0; return CUFFT_SUCCESS; }
 cufftResult cufftSetWorkArea(cufftHandle, void*) { return CUFFT_SUCCESS; }
-cufftResult cufftMakePlanMany(cufftHandle, int, int*, int*, int, int, int*, int, int, cufftType, int, size_t* n) {
-  *n = 1024;
-  return CUFFT_SUCCESS;
+cufftResult cufftMakePlanMany(cufftHandle h, int, int*, int*, int, int, int*, int, int, cufftType, int, size_t* n) {
+  *n = plan_bytes;
+  return plan_made(h);
 }
 cufftResult cufftPlanMany(cufftHandle* h, int, int*, int*, int, int, int*, int, int, cufftType, int) {
-  *h = 1;
-  return CUFFT_SUCCESS;
+  *h = ++last_plan;
+  return plan_made(*h);
 }
 cufftResult cufftPlan3d(cufftHandle* h, int, int, int, cufftType) { *h = 1; return CUFFT_SUCCESS; }
 cufftResult cufftExecR2C(cufftHandle, cufftReal*, cufftComplex*) { return CUFFT_SUCCESS; }
