@@ -156,6 +156,8 @@ struct gisapr_context {
   std::vector<IngestPlan> ingest;                      // at most kIngestPlans, and those that graphs hold
   unsigned long long ingest_calls = 0;
   cudaEvent_t ingest_done = nullptr;                   // the last call's transforms have run
+  unsigned long long ingest_stream = 0;                // and the id of its stream, if there was one
+  bool ingest_used = false;
   bool ingest_captured = false;                        // a graph holds the work area
   std::map<std::pair<int, int>, CorrTables> corr;      // (n, crop) -> twiddles
   DeviceBuffer atoms, bin_counts, bin_lists, proj_scratch, prep_scratch, proj_slices, proj_blocked, vfft_scratch;
@@ -298,10 +300,11 @@ int get_bins(gisapr_ctx ctx, int N, BinTable* out) {
 // The plans of ch x cw x n, kept with the context: making them took 0.4 ms of a
 // call and destroying them a wait for the stream. A fifth shape replaces the one
 // used longest ago. All plans share one work area (each of its own held as much as
-// a batch's spectra, twice for each of the shapes), so a call waits for the last
-// one, whatever its stream: the handle of a destroyed stream may come back for a
-// new one while the old one's work still runs. A capture cannot wait for work
-// outside it; whoever replays it orders it, and what it holds stays with the context.
+// a batch's spectra, twice for each of the shapes), so a call on another stream
+// waits for the last one (5 us of a call of 170). Streams are told apart by their
+// ids: a handle comes back when its stream is destroyed, whose work may still run.
+// A capture cannot wait for work outside it; whoever replays it orders it, and what
+// it holds stays with the context.
 int get_ingest_plan(gisapr_ctx ctx, int ch, int cw, int n, cudaStream_t st, bool capturing, IngestPlan** out) {
   if (ctx->ingest_done == nullptr)
     GISAPR_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->ingest_done, cudaEventDisableTiming), "cudaEventCreate(ingest)");
@@ -363,8 +366,16 @@ int get_ingest_plan(gisapr_ctx ctx, int ch, int cw, int n, cudaStream_t st, bool
     GISAPR_CHECK_CUDA(cudaMalloc(&b.ptr, p->work), "cudaMalloc(ingest transforms)");
     b.bytes = p->work;
   }
-  if (!capturing) GISAPR_CHECK_CUDA(cudaStreamWaitEvent(st, ctx->ingest_done, 0), "cudaStreamWaitEvent(ingest)");
-  if (capturing) p->captured = ctx->ingest_captured = true;
+  if (capturing) {
+    p->captured = ctx->ingest_captured = true;
+  } else {
+    unsigned long long id = 0;
+    GISAPR_CHECK_CUDA(cudaStreamGetId(st, &id), "cudaStreamGetId");
+    if (!ctx->ingest_used || id != ctx->ingest_stream)
+      GISAPR_CHECK_CUDA(cudaStreamWaitEvent(st, ctx->ingest_done, 0), "cudaStreamWaitEvent(ingest)");
+    ctx->ingest_used = true;
+    ctx->ingest_stream = id;
+  }
   p->used = ++ctx->ingest_calls;
   for (cufftHandle h : {p->forward, p->inverse}) {
     cufftSetStream(h, st);

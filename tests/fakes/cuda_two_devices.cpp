@@ -16,6 +16,7 @@ std::mutex guard;
 std::map<std::pair<int, const void*>, size_t> limits;
 int launched = 0, refused = 0, lowered = 0;
 int recorded = 0, waited = 0;  // events
+unsigned long long stream_id = 1;
 size_t held = 0, plan_held = 0, plan_bytes = 1024;  // device memory of the callers and of plans; what a plan takes
 std::map<void*, size_t> sizes;
 std::map<int, size_t> plans;  // handle -> work area of its own
@@ -49,6 +50,7 @@ int fake_refused() { return refused; }
 int fake_lowered() { return lowered; }
 int fake_recorded() { return recorded; }
 int fake_waited() { return waited; }
+void fake_new_stream() { ++stream_id; }  // the handles now belong to new streams
 long long fake_held() { return (long long)(held + plan_held); }
 void fake_plan_bytes(long long n) { plan_bytes = (size_t)n; }
 
@@ -59,6 +61,7 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 152; retu
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) { *s = cudaStreamCaptureStatusNone; return cudaSuccess; }
+cudaError_t cudaStreamGetId(cudaStream_t, unsigned long long* id) { *id = stream_id; return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { ++waited; return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = nullptr; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }

@@ -9,14 +9,16 @@ def call(n, size, stream=None, flags=7):
 """
 
 
-def test_every_call_waits_for_the_one_before(native_lib, tmp_path):
+def test_a_call_on_another_stream_waits_for_the_one_before(native_lib, tmp_path):
     """The work area is shared by all calls. A stream made where a destroyed one was has its handle, so an equal
     handle does not order the two."""
     run_on_fake(CALLS + r"""
-for k in range(1, 6):
-    call(4, 64, C.c_void_p(4096))
-    assert fake.fake_recorded() == k
-assert fake.fake_waited() >= 4, fake.fake_waited()
+for k in range(1, 11):
+    fake.fake_new_stream()
+    for again in range(2):
+        call(4, 64, C.c_void_p(4096))
+    assert fake.fake_recorded() == 2 * k
+    assert fake.fake_waited() >= k, fake.fake_waited()
 """, tmp_path)
 
 
