@@ -69,9 +69,11 @@ cudaError_t launch_restraint_poses(cudaStream_t, const float*, const float*, int
                                    void*, int*, int*, int);
 cudaError_t launch_restraint_reduce(cudaStream_t, float*, const unsigned char*, const int*, int, const int*,
                                     const int*, float, int*, int);
-cudaError_t launch_ingest_load(cudaStream_t, const float*, int, int, int, const int*, int, int, double*, int, int);
+size_t ingest_note_elems(int ch, int cw);
+cudaError_t launch_ingest_load(cudaStream_t, const float*, int, int, int, const int*, int, int, double*, int,
+                               const int*, const int*, int, const double*, int*, int, int);
 cudaError_t launch_ingest_spectrum(cudaStream_t, double2*, int, int, int, const int*, const int*, const double*, int,
-                                   int, const double*);
+                                   int, const double*, int*, int);
 cudaError_t launch_ingest_normalize(cudaStream_t, double*, int, int, int, int);
 cudaError_t launch_ingest_store(cudaStream_t, const double*, int, int, int, int, float*, int);
 int correlate_tc_max_psi();
@@ -162,6 +164,7 @@ struct gisapr_context {
   std::map<std::pair<int, int>, CorrTables> corr;      // (n, crop) -> twiddles
   DeviceBuffer atoms, bin_counts, bin_lists, proj_scratch, prep_scratch, proj_slices, proj_blocked, vfft_scratch;
   DeviceBuffer ingest_work;        // of all the kept transforms (they never run at once)
+  DeviceBuffer ingest_notes;       // on the tables of the call that runs
   DeviceBuffer proj_status;        // int: set to 1 by a projector plane wait that ran out
   unsigned proj_wait = 1u << 24;   // bound of that wait (attempts)
   int blocked_box = 0;  // box of the blocked spectrum gisapr_volume_spectrum_blocked last wrote (0: none)
@@ -519,6 +522,7 @@ int gisapr_context_destroy(gisapr_ctx ctx) {
   for (auto& p : ctx->ingest) { cufftDestroy(p.forward); cufftDestroy(p.inverse); }
   if (ctx->ingest_done != nullptr) cudaEventDestroy(ctx->ingest_done);
   cudaFree(ctx->ingest_work.ptr);
+  cudaFree(ctx->ingest_notes.ptr);
   for (auto& kv : ctx->bins) {
     cudaFree(kv.second.list); cudaFree(kv.second.off); cudaFree(kv.second.ptr); cudaFree(kv.second.count);
     cudaFree(kv.second.tw);
@@ -1064,21 +1068,30 @@ int gisapr_ingest_stack(gisapr_ctx ctx, void* stream, const float* images, int n
   const int ld = (flags & 5) ? 2 * (cw / 2 + 1) : cw;
   IngestPlan* plan = nullptr;
   bool capturing = false;
+  const int* const ptr = (flags & 1) ? bin_ptr : nullptr;
+  const double* const mask = (flags & 4) ? highpass_mask : nullptr;
   if (flags & 5) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     GISAPR_CHECK_CUDA(cudaStreamIsCapturing(st, &status), "cudaStreamIsCapturing");
     capturing = status != cudaStreamCaptureStatusNone;
     rc = get_ingest_plan(ctx, ch, cw, n, st, capturing, &plan);
     if (rc) return rc;
+    const size_t noted = ctx->ingest_notes.bytes;
+    rc = ensure(ctx, ctx->ingest_notes, ingest_note_elems(ch, cw) * sizeof(int), "cudaMalloc(table notes)");
+    if (rc) return rc;
+    if (ctx->ingest_notes.bytes != noted)
+      GISAPR_CHECK_CUDA(cudaMemsetAsync(ctx->ingest_notes.ptr, 0xff, ctx->ingest_notes.bytes, st), "cudaMemset(table notes)");
   }
-  GISAPR_CHECK_CUDA(launch_ingest_load(st, images, n, h, w, shifts, ch, cw, work, ld, ctx->sm_count), "ingest_load");
+  const int call = (int)(ctx->ingest_calls & 0x3fffffff);
+  GISAPR_CHECK_CUDA(launch_ingest_load(st, images, n, h, w, shifts, ch, cw, work, ld, ptr, bin_pix, n_bins, mask,
+                                       (int*)ctx->ingest_notes.ptr, call, ctx->sm_count),
+                    "ingest_load");
   if (flags & 5) {
     auto transforms = [&]() -> int {
       cufftResult r = cufftExecD2Z(plan->forward, (cufftDoubleReal*)work, (cufftDoubleComplex*)work);
       if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecD2Z failed");
-      GISAPR_CHECK_CUDA(launch_ingest_spectrum(st, (double2*)work, n, ch, cw, (flags & 1) ? bin_ptr : nullptr, bin_pix,
-                                               bin_count, n_bins, (flags & 2) ? 1 : 0,
-                                               (flags & 4) ? highpass_mask : nullptr),
+      GISAPR_CHECK_CUDA(launch_ingest_spectrum(st, (double2*)work, n, ch, cw, ptr, bin_pix, bin_count, n_bins,
+                                               (flags & 2) ? 1 : 0, mask, (int*)ctx->ingest_notes.ptr, call),
                         "ingest_spectrum");
       r = cufftExecZ2D(plan->inverse, (cufftDoubleComplex*)work, (cufftDoubleReal*)work);
       if (r != CUFFT_SUCCESS) return fail(GISAPR_ERR_CUFFT, "cufftExecZ2D failed");

@@ -31,9 +31,60 @@ namespace {
 constexpr int kIngestThreads = 256;
 constexpr int kSpectrumThreads = 512;
 
+// round(distance from the origin) of a pixel of the unshifted grid; y and x are
+// distances along the axes. No distance is half way between two integers.
+__device__ __forceinline__ int radius_bin(int y, int x) {
+  const long long d4 = 4 * ((long long)y * y + (long long)x * x);
+  int b = __float2int_rn(sqrtf(0.25f * (float)d4));
+  const long long up = 2LL * b + 1, down = 2LL * b - 1;
+  if (up * up < d4) ++b;
+  else if (b > 0 && down * down > d4) --b;
+  return b;
+}
+
+// What the spectrum kernel has to know of the caller's tables. bins_other and
+// mask_other hold the call's number if the bins are not the radial ones (in the
+// order of their lists or in number), if the mask is not its own mirror image.
+struct TableNotes {
+  const int* bin_ptr;      // null: no whitening
+  const int* bin_pix;
+  int n_bins;
+  const double* mask;      // or null
+  int call;
+  int* bins_other;
+  int* mask_other;
+  int* entry;              // [ch * cw] where a listed pixel stands in bin_pix
+};
+
+__device__ __forceinline__ int mirrored(int k, int n) { return k == 0 ? 0 : n - k; }
+
+// One pass over both tables by the threads of the load. An entry is where it
+// should be if it lies in the list of its pixel's radius.
+__device__ __forceinline__ void note_tables(const TableNotes& T, int ch, int cw, long long first, long long step) {
+  if (T.bin_ptr != nullptr) {
+    const int e0 = T.bin_ptr[0], e1 = T.bin_ptr[T.n_bins];
+    if (first == 0 && e1 - e0 != ch * cw) *T.bins_other = T.call;
+    for (long long e = e0 + first; e < e1; e += step) {
+      const int p = T.bin_pix[e];
+      if (p < 0 || p >= ch * cw) continue;
+      T.entry[p] = (int)e;
+      const int ky = p / cw, kx = p - ky * cw;
+      const int b = min(radius_bin(min(ky, ch - ky), min(kx, cw - kx)), T.n_bins - 1);
+      if (e < T.bin_ptr[b] || e >= T.bin_ptr[b + 1]) *T.bins_other = T.call;
+    }
+  }
+  if (T.mask != nullptr)
+    for (long long p = first; p < (long long)ch * cw; p += step) {
+      const int ky = (int)(p / cw), kx = (int)(p - (long long)ky * cw);
+      const double a = T.mask[p], b = T.mask[(size_t)mirrored(ky, ch) * cw + mirrored(kx, cw)];
+      if (__double_as_longlong(a) != __double_as_longlong(b)) *T.mask_other = T.call;
+    }
+}
+
 // ld: row stride of the result
 __global__ void ingest_load(const float* __restrict__ images, int n, int h, int w, const int* __restrict__ shifts,
-                            int ch, int cw, double* __restrict__ work, int ld) {
+                            int ch, int cw, double* __restrict__ work, int ld, TableNotes T) {
+  note_tables(T, ch, cw, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
   const long long total = (long long)n * ch * cw;
   const int y0 = h / 2 - ch / 2, x0 = w / 2 - cw / 2;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
@@ -151,7 +202,7 @@ __device__ __forceinline__ double sqrt_fp64(double e) {
 }
 
 struct SpectrumSteps {
-  const int* bin_ptr;       // null: no whitening. Radial bins: the bin of an axis pixel is its distance
+  const int* bin_ptr;       // null: no whitening
   const int* bin_pix;
   const double* bin_count;
   int n_bins;
@@ -159,7 +210,8 @@ struct SpectrumSteps {
   PlaneSums plane;
   int ramps;                // the axes' ramp transforms are kept in shared memory
   int amplitudes;           // the half spectrum's |F| are kept there too
-  const double* mask;       // [ch][cw] or null, symmetric under (ky, kx) -> (-ky, -kx) as a radial mask is
+  const double* mask;       // [ch][cw] or null
+  TableNotes notes;
 };
 
 // The steps of one image in its half spectrum [ch][cw/2 + 1], scaled by
@@ -170,14 +222,18 @@ struct SpectrumSteps {
 // memory an entry, 594 us for 500 spectra of 128 where this takes 475);
 // larger spectra are gathered. A pixel of
 // the full grid right of column cw/2 stands for its mirror, which has the same
-// magnitude, the same bin and the same mask: the columns that have a mirror
-// count twice.
-__global__ void __launch_bounds__(kSpectrumThreads) ingest_spectrum(double2* __restrict__ work, int ch, int cw,
-                                                                    SpectrumSteps P) {
-  extern __shared__ double s_div[];
-  __shared__ double red[kSpectrumThreads / 32];
+// magnitude and, where bins and mask are radial, the same bin and mask value: the
+// columns that have a mirror count twice.
+//
+// Bins and mask may be any (ANY: the bins are not the radial ones, or the mask is
+// not its own mirror image). The result of a step is the real part of its inverse
+// transform, that is, of a spectrum F(k) m(k) with real m the half of F(k) (m(k) +
+// m(-k)): the mean of a factor and its mirror image's stands for both, and a bin's
+// sum takes every pixel that it lists.
+template <bool ANY>
+__device__ __forceinline__ void spectrum_steps(double2* F, int ch, int cw, const SpectrumSteps& P, double* s_div,
+                                               double* red) {
   const int hc = cw / 2 + 1, pixels = ch * cw;
-  double2* F = work + (size_t)blockIdx.x * ch * hc;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const double inv = 1.0 / (double)pixels;
   auto doubled = [&](int kx) { return kx != 0 && 2 * kx != cw; };
@@ -203,12 +259,34 @@ __global__ void __launch_bounds__(kSpectrumThreads) ingest_spectrum(double2* __r
     }
     __syncthreads();
   }
+  // the divisor of a pixel by its entry in the lists (an entry left by an earlier
+  // call does not name the pixel), 1 if it has none
+  auto listed = [&](int ky, int kx) {
+    const int p = ky * cw + kx, e = P.notes.entry[p];
+    if (e < P.bin_ptr[0] || e >= P.bin_ptr[P.n_bins] || P.bin_pix[e] != p) return 1.0;
+    int lo = 0, hi = P.n_bins;  // the last bin that starts at e or before
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) / 2;
+      if (P.bin_ptr[mid] <= e) lo = mid;
+      else hi = mid;
+    }
+    return s_div[lo];
+  };
+  auto factor = [&](int ky, int kx) {
+    return P.bin_ptr == nullptr ? 1.0 : 0.5 * (listed(ky, kx) + listed(mirrored(ky, ch), mirrored(kx, cw)));
+  };
   double s2 = 0.0;  // this lane's part of the sum over the full grid of |V|^2, the axes added below
   for (int b = warp; P.bin_ptr != nullptr && b < P.n_bins; b += nw) {
     double s = 0.0, q = 0.0;
     for (int i = P.bin_ptr[b] + lane; i < P.bin_ptr[b + 1]; i += 32) {
-      const int p = P.bin_pix[i], ky = p / cw, kx = p - ky * cw;
-      if (kx >= hc) continue;
+      const int p = P.bin_pix[i];
+      int ky = p / cw, kx = p - ky * cw;
+      const bool right = kx >= hc;
+      if (right) {
+        if (!ANY) continue;
+        ky = mirrored(ky, ch);
+        kx = cw - kx;
+      }
       double e, a;
       if (P.amplitudes) {
         a = s_amp[ky * hc + kx];
@@ -218,26 +296,27 @@ __global__ void __launch_bounds__(kSpectrumThreads) ingest_spectrum(double2* __r
         e = fma(f.x, f.x, f.y * f.y);
         a = sqrt_fp64(e);
       }
-      s += doubled(kx) ? 2.0 * a : a;
-      if (ky != 0 && kx != 0) q += doubled(kx) ? 2.0 * e : e;
+      s += !ANY && doubled(kx) ? 2.0 * a : a;
+      if (!ANY && ky != 0 && kx != 0) q += doubled(kx) ? 2.0 * e : e;
     }
     s = warp_sum_d(s);
     const double d = (b == 0 || P.bin_count[b] <= 0.0) ? 1.0 : 1.0 / (s / P.bin_count[b]);
-    s2 = fma(d * d, q, s2);
+    if (!ANY) s2 = fma(d * d, q, s2);
     if (lane == 0) s_div[b] = d;
   }
   __syncthreads();
   auto divisor = [&](int bin) { return P.bin_ptr != nullptr ? s_div[min(bin, P.n_bins - 1)] : 1.0; };
   auto axis_y = [&](int ky) { return min(ky, ch - ky); };
+  auto axis_divisor = [&](int ky, int kx) { return ANY ? factor(ky, kx) : divisor(ky == 0 ? kx : axis_y(ky)); };
   double pa = 0.0, pb = 0.0, pc = 0.0, scale = inv;
   bool centre = false;
   if (P.normalize) {
-    if (P.bin_ptr == nullptr) {
+    if (ANY || P.bin_ptr == nullptr) {
       for (long long t = threadIdx.x; t < (long long)ch * hc; t += blockDim.x) {
         const int ky = (int)(t / hc), kx = (int)(t - (long long)ky * hc);
         if (ky == 0 || kx == 0) continue;
         const double2 f = F[t];
-        const double e = fma(f.x, f.x, f.y * f.y);
+        const double d = ANY ? factor(ky, kx) : 1.0, e = d * d * fma(f.x, f.x, f.y * f.y);
         s2 += doubled(kx) ? 2.0 * e : e;
       }
     }
@@ -245,16 +324,16 @@ __global__ void __launch_bounds__(kSpectrumThreads) ingest_spectrum(double2* __r
     double J = 0.0, K = 0.0;
     for (int kx = threadIdx.x; kx < hc; kx += blockDim.x) {
       const double2 f = F[kx], x = ramp_x(kx);
-      const double v = (f.x * x.x + f.y * x.y) * divisor(kx);
+      const double v = (f.x * x.x + f.y * x.y) * axis_divisor(0, kx);
       J += doubled(kx) ? 2.0 * v : v;
     }
     for (int ky = threadIdx.x; ky < ch; ky += blockDim.x) {
       const double2 f = F[(size_t)ky * hc], y = ramp_y(ky);
-      K += (f.x * y.x + f.y * y.y) * divisor(axis_y(ky));
+      K += (f.x * y.x + f.y * y.y) * axis_divisor(ky, 0);
     }
     J = block_sum_d(J, red) / (double)cw;
     K = block_sum_d(K, red) / (double)ch;
-    const double L = F[0].x * divisor(0);
+    const double L = F[0].x * axis_divisor(0, 0);
     plane_fit(P.plane, J, K, L, pa, pb, pc);
   }
   // value of the plane-free spectrum on an axis
@@ -279,12 +358,12 @@ __global__ void __launch_bounds__(kSpectrumThreads) ingest_spectrum(double2* __r
   if (P.normalize) {
     for (int k = threadIdx.x; k < hc + ch - 1; k += blockDim.x) {
       const int kx = k < hc ? k : 0, ky = k < hc ? 0 : k - hc + 1;
-      const double2 v = axis_value(ky, kx, divisor(k < hc ? kx : axis_y(ky)));
+      const double2 v = axis_value(ky, kx, axis_divisor(ky, kx));
       const double e = fma(v.x, v.x, v.y * v.y);
       s2 += doubled(kx) ? 2.0 * e : e;
     }
     s2 = block_sum_d(s2, red) * inv;  // sum of v^2 over the pixels
-    const double ave = axis_value(0, 0, divisor(0)).x * inv;
+    const double ave = axis_value(0, 0, axis_divisor(0, 0)).x * inv;
     const double sd = sqrt(__dsub_rn(s2 * inv, __dmul_rn(ave, ave)));
     if (sd > 0.0) {
       scale = inv / sd;
@@ -295,6 +374,7 @@ __global__ void __launch_bounds__(kSpectrumThreads) ingest_spectrum(double2* __r
   auto finish = [&](int ky, int kx, double d) {
     const size_t o = (size_t)ky * hc + kx;
     double m = P.mask != nullptr ? P.mask[(size_t)ky * cw + kx] * scale : scale;
+    if (ANY && P.mask != nullptr) m = 0.5 * (m + P.mask[(size_t)mirrored(ky, ch) * cw + mirrored(kx, cw)] * scale);
     double2 v;
     if (ky == 0 || kx == 0) {
       v = axis_value(ky, kx, d);
@@ -305,7 +385,12 @@ __global__ void __launch_bounds__(kSpectrumThreads) ingest_spectrum(double2* __r
     }
     F[o] = make_double2(v.x * m, v.y * m);
   };
-  if (P.amplitudes) {
+  if (ANY) {
+    for (long long t = threadIdx.x; t < (long long)ch * hc; t += blockDim.x) {
+      const int ky = (int)(t / hc), kx = (int)(t % hc);
+      finish(ky, kx, factor(ky, kx));
+    }
+  } else if (P.amplitudes) {
     // in order; the bin by its definition, round(distance): a distance of an
     // integer d2 < 2^16 is at least 2^-11 from a half, float32's square root
     // within 2^-15 of it
@@ -327,6 +412,17 @@ __global__ void __launch_bounds__(kSpectrumThreads) ingest_spectrum(double2* __r
   }
 }
 
+__global__ void __launch_bounds__(kSpectrumThreads) ingest_spectrum(double2* __restrict__ work, int ch, int cw,
+                                                                    SpectrumSteps P) {
+  extern __shared__ double s_div[];
+  __shared__ double red[kSpectrumThreads / 32];
+  double2* F = work + (size_t)blockIdx.x * ch * (cw / 2 + 1);
+  const bool any = (P.bin_ptr != nullptr && *P.notes.bins_other == P.notes.call) ||
+                   (P.mask != nullptr && *P.notes.mask_other == P.notes.call);
+  if (any) spectrum_steps<true>(F, ch, cw, P, s_div, red);
+  else spectrum_steps<false>(F, ch, cw, P, s_div, red);
+}
+
 __global__ void ingest_store(const double* __restrict__ work, long long total, int cw, int ld, float* __restrict__ out) {
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -343,6 +439,14 @@ int grid_of(long long total, int sm_count) {
 
 }  // namespace
 
+// ints of the notes on a call's tables
+size_t ingest_note_elems(int ch, int cw) { return 2 + (size_t)ch * cw; }
+
+static TableNotes table_notes(const int* bin_ptr, const int* bin_pix, int n_bins, const double* mask, int* notes,
+                              int call) {
+  return TableNotes{bin_ptr, bin_pix, n_bins, mask, call, notes, notes + 1, notes + 2};
+}
+
 // sums over the pixel grid of x^2, xy, x, y^2, y and 1, exact in integers
 static PlaneSums plane_sums(int ch, int cw) {
   const long long h = ch, w = cw;
@@ -353,15 +457,16 @@ static PlaneSums plane_sums(int ch, int cw) {
 }
 
 cudaError_t launch_ingest_load(cudaStream_t st, const float* images, int n, int h, int w, const int* shifts, int ch,
-                               int cw, double* work, int ld, int sm_count) {
-  ingest_load<<<grid_of((long long)n * ch * cw, sm_count), kIngestThreads, 0, st>>>(images, n, h, w, shifts, ch,
-                                                                                   cw, work, ld);
+                               int cw, double* work, int ld, const int* bin_ptr, const int* bin_pix, int n_bins,
+                               const double* mask, int* notes, int call, int sm_count) {
+  ingest_load<<<grid_of((long long)n * ch * cw, sm_count), kIngestThreads, 0, st>>>(
+      images, n, h, w, shifts, ch, cw, work, ld, table_notes(bin_ptr, bin_pix, n_bins, mask, notes, call));
   return cudaGetLastError();
 }
 
 cudaError_t launch_ingest_spectrum(cudaStream_t st, double2* work, int n, int ch, int cw, const int* bin_ptr,
                                    const int* bin_pix, const double* bin_count, int n_bins, int normalize,
-                                   const double* mask) {
+                                   const double* mask, int* notes, int call) {
   const size_t bins = bin_ptr != nullptr ? (size_t)n_bins * sizeof(double) : 0;
   const size_t ramps = normalize ? (size_t)(cw / 2 + 1 + ch) * sizeof(double) : 0;
   const bool keep = bins + ramps <= 96 * 1024;  // else the ramps are computed where they are used
@@ -371,7 +476,8 @@ cudaError_t launch_ingest_spectrum(cudaStream_t st, double2* work, int n, int ch
   static SmemLimit limit;
   const cudaError_t e = allow_smem(ingest_spectrum, smem, limit);
   if (e != cudaSuccess) return e;
-  const SpectrumSteps P{bin_ptr, bin_pix, bin_count, n_bins, normalize, plane_sums(ch, cw), keep && normalize ? 1 : 0, hold ? 1 : 0, mask};
+  const SpectrumSteps P{bin_ptr, bin_pix, bin_count, n_bins, normalize, plane_sums(ch, cw), keep && normalize ? 1 : 0, hold ? 1 : 0, mask,
+                        table_notes(bin_ptr, bin_pix, n_bins, mask, notes, call)};
   ingest_spectrum<<<n, kSpectrumThreads, smem, st>>>(work, ch, cw, P);
   return cudaGetLastError();
 }

@@ -342,11 +342,13 @@ int gisapr_score_sum_batch(void* stream, const int* local_ptr, const float* peak
  * (zero fill) is cropped to the centred ch x cw window, then flags select:
  * 1 = divide by the radial mean amplitude spectrum (getSpectrum_divideBy
  * Spectrum; bin tables: CSR bin_ptr[n_bins + 1] / bin_pix of row-major pixel
- * indices of the unshifted transform grid per bin round(centred radius),
- * bin_count = pixels per bin), 2 = least-squares plane removal and mean/sigma
- * normalisation (normalize), 4 = high-pass by highpass_mask (ch*cw doubles,
- * unshifted order, radial). Bins and mask depend on the centred radius alone:
- * the steps run in the half spectrum of real images. The context keeps the
+ * indices of the unshifted transform grid per bin, the reference's being
+ * round(centred radius); bin_count = pixels per bin; a pixel stands in one bin
+ * at most), 2 = least-squares plane removal and mean/sigma normalisation
+ * (normalize), 4 = high-pass by highpass_mask (ch*cw doubles, unshifted order).
+ * The steps run in the half spectrum of real images; bins that are not the
+ * radial ones, and a mask that is not its own mirror image, take a slower way
+ * through it. The context keeps the
  * transform plans of the last four (ch, cw, n) and one work area for all of
  * them, as large as the largest needs; one above 1 GB is given back after the
  * call, which then waits for it.

@@ -23,8 +23,8 @@ for k in range(1, 11):
 
 
 def test_kept_transforms_share_one_work_area(native_lib, tmp_path):
-    """Calls of many shapes leave one work area behind, as large as the largest took, whatever the order; one above
-    1 GB is gone after the call, and so is everything with the context."""
+    """Calls of many shapes leave one work area behind, as large as the largest took, whatever the order (and a few kB
+    of notes on their tables); one above 1 GB is gone after the call, and so is everything with the context."""
     run_on_fake(CALLS + r"""
 fake.fake_held.restype = C.c_longlong
 fake.fake_plan_bytes.argtypes = [C.c_longlong]
@@ -35,14 +35,14 @@ for turn in range(3):
     for n, size, take in ((5, 64, 100), (6, 64, 120), (7, 32, 40), (8, 48, 300), (9, 50, 20), (10, 64, 200)):
         fake.fake_plan_bytes(take * MB)
         call(n, size)
-        assert fake.fake_held() - empty <= 300 * MB, (turn, n, (fake.fake_held() - empty) // MB)
+        assert fake.fake_held() - empty <= 301 * MB, (turn, n, (fake.fake_held() - empty) // MB)
 fake.fake_plan_bytes(3000 * MB)
 call(11, 64)
-assert fake.fake_held() - empty <= 300 * MB, (fake.fake_held() - empty) // MB
+assert fake.fake_held() - empty <= 301 * MB, (fake.fake_held() - empty) // MB
 fake.fake_plan_bytes(100 * MB)
 call(12, 64)
 call(12, 64, flags=1)
-assert fake.fake_held() - empty <= 300 * MB
+assert fake.fake_held() - empty <= 301 * MB
 ok(lib.gisapr_context_destroy(context), "destroy")
 assert fake.fake_held() == 0, fake.fake_held()
 """, tmp_path)
