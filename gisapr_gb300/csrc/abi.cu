@@ -451,6 +451,19 @@ int tuned_cluster(gisapr_ctx ctx, int n) {
   return it == ctx->tune_corr_cluster.end() ? 0 : it->second;
 }
 
+// CTAs per particle of the general correlation (0: its default), which holds its
+// columns of every psi spectrum in shared memory. A tuned number that they do not
+// fit gives way to the default: it may have been tuned for a window that the
+// register form takes, which has no such limit.
+int plain_cluster(gisapr_ctx ctx, int n, int n_psi, int crop, int* cluster) {
+  constexpr size_t kMost = 227 * 1024;
+  *cluster = tuned_cluster(ctx, n);
+  if (correlate_smem_bytes(n, n_psi, crop, *cluster) > kMost) *cluster = 0;
+  if (correlate_smem_bytes(n, n_psi, crop, *cluster) > kMost)
+    return fail(GISAPR_ERR_UNSUPPORTED, "too many psi angles for the shared-memory particle slice");
+  return GISAPR_OK;
+}
+
 // Boxes are powers of two from 32 to 256, or 96 and 192 (3 * 2^k: the
 // shared-memory transforms run a radix-3 pass over radix-2 sub-transforms).
 int check_box(int box) {
@@ -802,10 +815,6 @@ int gisapr_correlate_batch_subset(gisapr_ctx ctx, void* stream, const float* ban
     return fail(GISAPR_ERR_UNSUPPORTED, "correlation size must be a multiple of 16 in [32, 256]");
   if (crop < 2 || crop > 16 || crop % 2 != 0 || crop > n)
     return fail(GISAPR_ERR_UNSUPPORTED, "crop must be even, 2..16 and <= n");
-  const int cluster = tuned_cluster(ctx, n);
-  const size_t smem = correlate_smem_bytes(n, n_psi, crop, cluster);
-  if (smem > 227 * 1024)
-    return fail(GISAPR_ERR_UNSUPPORTED, "too many psi angles for the shared-memory particle slice");
   int rc = set_device(ctx);
   if (rc) return rc;
   CorrTables t;
@@ -815,9 +824,13 @@ int gisapr_correlate_batch_subset(gisapr_ctx ctx, void* stream, const float* ban
   bool taken;
   GISAPR_CHECK_CUDA(launch_correlate_rows((cudaStream_t)stream, (const float2*)bank, (const float2*)stack,
                                           local_ptr, local_idx, n_particles, n_psi, n, crop, t.outer, t.col,
-                                          out_score, out_y, out_x, n_cand, bank_stride, nnz, cluster, subset, ctx->sm_count, &taken),
+                                          out_score, out_y, out_x, n_cand, bank_stride, nnz, tuned_cluster(ctx, n), subset,
+                                          ctx->sm_count, &taken),
                     "correlate");
   if (taken) return GISAPR_OK;
+  int cluster;
+  rc = plain_cluster(ctx, n, n_psi, crop, &cluster);
+  if (rc) return rc;
   GISAPR_CHECK_CUDA(launch_correlate_plain((cudaStream_t)stream, (const float2*)bank, (const float2*)stack,
                                            local_ptr, local_idx, n_particles, n_psi, n, crop, t.outer, t.col,
                                            out_score, out_y, out_x, n_cand, bank_stride, nnz, cluster, subset),
@@ -844,10 +857,6 @@ int gisapr_correlate(gisapr_ctx ctx, void* stream, const float* bank, const floa
     return fail(GISAPR_ERR_UNSUPPORTED, "correlation size must be a multiple of 16 in [32, 256]");
   if (crop < 2 || crop > 16 || crop % 2 != 0 || crop > n)
     return fail(GISAPR_ERR_UNSUPPORTED, "crop must be even, 2..16 and <= n");
-  const int cluster = tuned_cluster(ctx, n);
-  const size_t smem = correlate_smem_bytes(n, n_psi, crop, cluster);
-  if (smem > 227 * 1024)
-    return fail(GISAPR_ERR_UNSUPPORTED, "too many psi angles for the shared-memory particle slice");
   int rc = set_device(ctx);
   if (rc) return rc;
   CorrTables t;
@@ -856,9 +865,12 @@ int gisapr_correlate(gisapr_ctx ctx, void* stream, const float* bank, const floa
   bool taken;
   GISAPR_CHECK_CUDA(launch_correlate_rows((cudaStream_t)stream, (const float2*)bank, (const float2*)stack,
                                           local_ptr, local_idx, n_particles, n_psi, n, crop, t.outer, t.col,
-                                          out_score, out_y, out_x, 1, 0, 0, cluster, nullptr, ctx->sm_count, &taken),
+                                          out_score, out_y, out_x, 1, 0, 0, tuned_cluster(ctx, n), nullptr, ctx->sm_count, &taken),
                     "correlate");
   if (taken) return GISAPR_OK;
+  int cluster;
+  rc = plain_cluster(ctx, n, n_psi, crop, &cluster);
+  if (rc) return rc;
   GISAPR_CHECK_CUDA(launch_correlate_plain((cudaStream_t)stream, (const float2*)bank, (const float2*)stack,
                                            local_ptr, local_idx, n_particles, n_psi, n, crop, t.outer, t.col,
                                            out_score, out_y, out_x, 1, 0, 0, cluster, nullptr),

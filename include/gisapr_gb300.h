@@ -245,7 +245,8 @@ int gisapr_score_sum_subset(void* stream, const int* local_ptr, const float* pea
  *   GISAPR_TUNE_CORR_CLUSTER: CTAs per particle (thread-block cluster size,
  *     1..8; 0 = the default) of gisapr_correlate and gisapr_correlate_batch
  *     at correlation size ``size``. Results do not depend on it beyond
- *     float32 summation order of the cluster's partial maps.
+ *     float32 summation order of the cluster's partial maps. A number that
+ *     the shared memory does not allow gives way to the default.
  *   GISAPR_TUNE_TC_A_STAGES / GISAPR_TUNE_TC_B_STAGES: shared-memory ring
  *     depths of the tensor-core correlation at particle size ``size`` (A:
  *     bulk-copied template rows, 2..8; B: built particle rows, 2..3; 0 =
