@@ -32,6 +32,7 @@ SIGNATURES = {
     "gisapr_packed_ctf": [_p, _p, _p, _p, _i, _p, _p, _p, _p, _i, _f, _f, _f, _f, _f, _p],
     "gisapr_prepare_particles": [_p, _p, _p, _i, _i, _p, _p, _p, _p, _i, _i, _p],
     "gisapr_correlate": [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _p, _p, _p],
+    "gisapr_correlate_form": [_i, _i, C.POINTER(_i)],
     "gisapr_particle_results": [_p, _p, _p, _p, _p, _i, _i, _p, _p, _p, _p, _p, _p],
     "gisapr_score_sum": [_p, _p, _p, _i, _p],
     "gisapr_correlate_batch": [_p, _p, _p, C.c_longlong, _i, _p, _p, _p, _i, _i, _i, _i, _i, _p, _p, _p],
@@ -117,6 +118,15 @@ def stream_of(device) -> C.c_void_p:
 TUNE_CORR_CLUSTER = 1  # gisapr_set_tuning keys (include/gisapr_gb300.h)
 TUNE_TC_A_STAGES = 2
 TUNE_TC_B_STAGES = 3
+CORRELATE_GENERAL, CORRELATE_ROWS = 1, 2  # gisapr_correlate_form
+
+
+def correlate_form(n: int, crop: int) -> int:
+    """The kernel that the plain correlation runs at size ``n`` and window ``crop``."""
+    form = C.c_int()
+    call("gisapr_correlate_form", int(n), int(crop), C.byref(form))
+    return form.value
+
 
 # Process-wide launch-shape settings, (key, size) -> value, applied to every
 # native context at creation (and to this thread's contexts when changed);

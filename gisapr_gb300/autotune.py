@@ -4,8 +4,8 @@ Four launch choices decide a batch's speed for a given box, crop, psi count
 and particle set, and the best values depend on the GPU:
 
 * the thread-block cluster size of the plain FP32 correlation (CTAs that
-  split one particle's packed columns; each holds its columns of every psi
-  spectrum in shared memory), 1..8;
+  split one particle's packed columns): 1..8, or 0, the kernel's own choice by
+  the number of particles, which stands unless another is clearly faster;
 * the candidates per tensor-core launch: a 128-row MMA tile holds
   128 // ceil8(candidates) whole directions, so the chunk size sets how many
   directions share a tile (the tile shape) and how many tiles a particle
@@ -20,10 +20,10 @@ and particle set, and the best values depend on the GPU:
 
 ``Autotuner.tune`` times the batched correlation stage (CUDA events, best of
 a few runs on the job's own data) for every valid value, keeps the fastest,
-and caches the result per (GPU, size, crop, psi count, particle count
-bucket, batch size) in a JSON file. The reference has no autotuner (its
-launch shapes are fixed in the torch code); these choices change launch
-shapes only, not the algorithm.
+and caches the result per (GPU, size, crop, psi count, particle count bucket,
+batch size, correlation kernel) in a JSON file. The reference has no
+autotuner (its launch shapes are fixed in the torch code); these choices
+change launch shapes only, not the algorithm.
 """
 from __future__ import annotations
 
@@ -42,7 +42,7 @@ CLUSTER_CHOICES = (1, 2, 3, 4, 5, 6, 8)
 CHUNK_CHOICES = (16, 32, 64, 128)
 RING_CHOICES = ((4, 2), (3, 2), (6, 2), (4, 3))  # (A, B) ring depths; the first is the kernel's default
 LANE_CHOICES = (1, 2, 3)
-SMEM_LIMIT = 227 * 1024
+NOISE = 0.02  # runs of one launch shape differ by up to this
 
 
 def default_cache_path() -> Path:
@@ -50,15 +50,6 @@ def default_cache_path() -> Path:
     if env:
         return Path(env)
     return Path.home() / ".cache" / "gisapr_gb300" / "tuning.json"
-
-
-def plain_smem_bytes(n: int, n_psi: int, crop: int, cluster: int) -> int:
-    """Shared memory of one CTA of the plain correlation (matches the kernel's carve-up)."""
-    h = n // 2 + 1
-    cw = -(-h // cluster)
-    k_group, k_local = 4, 16
-    return (n_psi * n * cw * 8 + k_group * n_psi * crop * cw * 8 + (n // 16) * crop * 8 + cw * crop * 8
-            + k_local * n_psi * crop * crop * 4)
 
 
 @dataclass
@@ -91,7 +82,9 @@ class Autotuner:
         import torch
         name = torch.cuda.get_device_name(job.device).replace("|", "/")
         bucket = 2 ** int(round(math.log2(max(1, len(job.records)))))
-        return f"{name}|n={job.cfg.new_box}|crop={job.cfg.crop}|psi={job.n_psi}|particles~{bucket}|cand={n_cand}"
+        form = nat.correlate_form(job.cfg.new_box, job.cfg.crop)
+        return (f"{name}|n={job.cfg.new_box}|crop={job.cfg.crop}|psi={job.n_psi}|particles~{bucket}|cand={n_cand}"
+                f"|kernel={form}")
 
     def _load(self) -> dict:
         try:
@@ -154,17 +147,19 @@ class Autotuner:
             r.apply()
             return r
         poses = list(syn.candidate_poses(n_cand, 1234, 5.0, 3.0))
-        nb, crop, n_psi = job.cfg.new_box, job.cfg.crop, job.n_psi
+        nb, crop = job.cfg.new_box, job.cfg.crop
         times: Dict[str, float] = {}
         best_k, best_t = 0, math.inf
         ctx = nat.Context.for_device(job.device)
-        for k in clusters:
-            if plain_smem_bytes(nb, n_psi, crop, k) > SMEM_LIMIT or k > nb // 2 + 1:
+        # Automatic first, where it is a choice of its own: the general kernel's is one of the others.
+        auto = nat.correlate_form(nb, crop) == nat.CORRELATE_ROWS
+        for k in ((0,) if auto else ()) + tuple(k for k in clusters if k > 0):
+            if k > nb // 2 + 1:
                 continue
             nat.call("gisapr_set_tuning", ctx.handle, nat.TUNE_CORR_CLUSTER, nb, k)
             t = self._time_correlate(job, n_cand, "fp32", poses)
             times[f"plain_cluster_{k}"] = t
-            if t < best_t:
+            if t < best_t * (1.0 - NOISE if auto and best_k == 0 else 1.0):
                 best_k, best_t = k, t
         nat.call("gisapr_set_tuning", ctx.handle, nat.TUNE_CORR_CLUSTER, nb, best_k)
         best_c = min(128, n_cand)

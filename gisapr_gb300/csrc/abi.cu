@@ -57,6 +57,7 @@ cudaError_t launch_correlate_plain(cudaStream_t, const float2*, const float2*, c
 cudaError_t launch_correlate_rows(cudaStream_t, const float2*, const float2*, const int*,
                                    const int*, int, int, int, int, const float2*, const float2*,
                                    float*, int*, int*, int, long long, int, int, const unsigned char*, int, bool*);
+bool correlate_rows_takes(int n, int crop);
 cudaError_t launch_particle_results(cudaStream_t, const int*, const float*, const int*, const int*,
                                     int, int, int*, int*, float*, int*, int*, float*, int, const unsigned char*);
 cudaError_t launch_score_sum(cudaStream_t, const int*, const float*, int, double*, int, const unsigned char*);
@@ -875,6 +876,12 @@ int gisapr_correlate(gisapr_ctx ctx, void* stream, const float* bank, const floa
                                            local_ptr, local_idx, n_particles, n_psi, n, crop, t.outer, t.col,
                                            out_score, out_y, out_x, 1, 0, 0, cluster, nullptr),
                     "correlate");
+  return GISAPR_OK;
+}
+
+int gisapr_correlate_form(int n, int crop, int* form) {
+  if (!form) return fail(GISAPR_ERR_ARGUMENT, "form is NULL");
+  *form = correlate_rows_takes(n, crop) ? GISAPR_CORRELATE_ROWS : GISAPR_CORRELATE_GENERAL;
   return GISAPR_OK;
 }
 

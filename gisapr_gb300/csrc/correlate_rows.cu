@@ -418,6 +418,11 @@ cudaError_t launch_size(const RowsParams& P, int n, int sm_count, cudaStream_t s
 
 }  // namespace
 
+// Whether this form has the size and window.
+bool correlate_rows_takes(int n, int crop) {
+  return (n == 64 || n == 96 || n == 128 || n == 192 || n == 256) && crop >= 8 && crop <= 16 && crop % 2 == 0;
+}
+
 // *taken: this form has the size and window, and was launched. Templates must
 // start on 16 bytes.
 cudaError_t launch_correlate_rows(cudaStream_t st, const float2* bank, const float2* stack, const int* local_ptr,
@@ -426,7 +431,7 @@ cudaError_t launch_correlate_rows(cudaStream_t st, const float2* bank, const flo
                                   int* out_x, int n_cand, long long bank_stride, int nnz, int cluster,
                                   const unsigned char* subset, int sm_count, bool* taken) {
   *taken = false;
-  if (n_particles <= 0 || n_cand <= 0) return cudaSuccess;
+  if (n_particles <= 0 || n_cand <= 0 || !correlate_rows_takes(n, crop)) return cudaSuccess;
   if (reinterpret_cast<uintptr_t>(bank) % 16 != 0 || bank_stride % 2 != 0) return cudaSuccess;
   RowsParams P{bank, stack, local_ptr, local_idx, tw_outer, tw_col, out_score, out_y, out_x, n_particles, n_psi, cluster,
                n_cand, bank_stride, nnz, subset, 0};

@@ -240,6 +240,16 @@ int gisapr_score_sum_subset(void* stream, const int* local_ptr, const float* pea
                             const unsigned char* subset, double* out);
 
 /*
+ * The kernel that the plain correlation runs at size n and window crop (for
+ * templates that start on 16 bytes): the one with the particle's spectrum in
+ * registers, whose default cluster size follows the number of particles, or the
+ * general one, whose default follows n alone. A new kernel gets a new number, so
+ * launch shapes tuned for one are not taken for another's.
+ */
+enum { GISAPR_CORRELATE_GENERAL = 1, GISAPR_CORRELATE_ROWS = 2 };
+int gisapr_correlate_form(int n, int crop, int* form);
+
+/*
  * Launch-shape knobs of a context per transform size, chosen by the
  * autotuner (gisapr_gb300/autotune.py); no counterpart in the reference.
  *   GISAPR_TUNE_CORR_CLUSTER: CTAs per particle (thread-block cluster size,
