@@ -11,7 +11,8 @@ moves the chain with the reference's float32 row-vector rotation about its
 mean (v8:33-45, on the host, as the reference computes it), and the moved
 chain's density is met with mask and distance transform voxel by voxel as it
 is computed: overlap voxels are counted and the minimum squared distance
-taken, with no volume in between. ``evaluate_many`` scores a list of poses
+taken, with no volume in between (but for a threshold below zero, where voxels
+that no atom reaches count as well). ``evaluate_many`` scores a list of poses
 with one upload of every pose's coordinates, the splat of up to 32 poses in
 one launch, and one read-back of all results.
 
@@ -21,6 +22,7 @@ same splat as the scoring path. There is no CPU path.
 from __future__ import annotations
 
 import argparse
+import functools
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -95,10 +97,14 @@ class GeometryRestraint:
                  nat.ptr(self.mainbody_mask), nat.ptr(self.mainbody_d2), nat.ptr(scratch))
         del rest, scratch
         self.has_mainbody = bool(torch.count_nonzero(self.mainbody_mask).item())
-        self._volume = torch.zeros((n, n, n), dtype=torch.float32, device=self.device)
         self._empty_chain_distance: Optional[float] = None
 
     # -------------------------------------------------------------------
+    @functools.cached_property
+    def _volume(self) -> torch.Tensor:
+        """Density of one pose, all zeros between calls; made by the first call that needs it."""
+        return torch.zeros((self.boxsize,) * 3, dtype=torch.float32, device=self.device)
+
     @property
     def mainbody_distance(self) -> torch.Tensor:
         """Distance transform in voxels (float64), as the reference keeps it."""
