@@ -531,14 +531,9 @@ static size_t general_smem_bytes(int N, int n_bins) {
 namespace {
 
 // Columns a warp transforms per pass-A round: G = 32 / (N/16) lines, two
-// per column (even and odd rows of the 2N grid). The even line of column c
-// is transformed in place in plane column c (which then receives the
-// column's output); only the odd lines need staging.
+// per column (even and odd rows of the 2N grid).
 template <int N>
 __host__ __device__ constexpr int pass_a_cols() { return 16 / (N / 16); }
-
-
-
 
 // The half-volume spectrum in the blocked layout the slice gather reads:
 // centred order along z and y, cut into blocks of 2 (z) x 4 (y) x 2 (x)
@@ -550,12 +545,6 @@ constexpr int kBZ = 2, kBY = 4, kBX = 2, kBE = kBZ * kBY * kBX;
 
 template <int N>
 __host__ __device__ constexpr int blocked_x() { return (N + 1 + kBX - 1) / kBX; }
-
-template <int N>
-__device__ __forceinline__ int blocked_off(int z, int y, int x) {
-  constexpr int YB = 2 * N / kBY, XB = blocked_x<N>();
-  return (((z / kBZ) * YB + y / kBY) * XB + x / kBX) * kBE + ((z % kBZ) * kBY + y % kBY) * kBX + x % kBX;
-}
 
 template <int N>
 __global__ void __launch_bounds__(256) spectrum_blocked(const float2* __restrict__ spectrum,
