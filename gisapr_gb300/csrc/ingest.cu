@@ -184,23 +184,6 @@ __device__ __forceinline__ double ramp_imag(int k, int n) {
   return 0.5 * (double)n * (c / s);
 }
 
-// Square root in eight FP64 operations: Goldschmidt's iteration from the
-// hardware estimate of 1 / sqrt(e) and one correction by the exact remainder
-// (Markstein, IBM RS/6000, 1990), within 2^-52 of the value. The general square
-// root took half of this kernel at GB300's FP64 rate.
-__device__ __forceinline__ double sqrt_fp64(double e) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(e));
-  double g = e * y, h = 0.5 * y;
-  const double r = fma(-g, h, 0.5);
-  g = fma(g, r, g);
-  h = fma(h, r, h);
-  const double r2 = fma(-g, h, 0.5);
-  g = fma(g, r2, g);
-  g = fma(fma(-g, g, e), h, g);
-  return e > 0.0 ? g : e;  // 0 and NaN as they are
-}
-
 struct SpectrumSteps {
   const int* bin_ptr;       // null: no whitening
   const int* bin_pix;
