@@ -23,7 +23,7 @@
 // rate, and they run at that limit. Real data in place of complex and one pair
 // of transforms in place of two (whitening and high-pass each had its own) cut
 // them to a quarter. Measured on GB300, 500 images of 256 cropped to 128,
-// whitened and high-passed: 5.47 -> 1.88 ms (1.25 of it the transforms).
+// whitened and high-passed: 5.47 -> 1.89 ms (1.25 of it the transforms).
 #include "common.cuh"
 
 namespace {

@@ -45,7 +45,8 @@ GISAPR_DEV float small_to_float(int i) {  // 0 <= i < 2^23, FP32 pipe
 // Packed product for a packed sum. A plain one may be fused into the sum (the
 // assembler does), and then neither the floor and the fraction of a coordinate nor
 // the sample's terms have the roundings they should; adding zero rounds nothing
-// and leaves only a sum of sums.
+// and leaves only a sum of sums (749 us for 6,000 spectra of box 128, 744 with
+// plain products).
 GISAPR_DEV float2 mul_alone(float2 a, float2 b) { return fma2(a, b, dup2(0.0f)); }
 
 // Pixels (2 q, j) and (2 q + 1, j) of the image rotated by ``ps`` (cos, sin, offset
